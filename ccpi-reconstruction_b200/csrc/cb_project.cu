@@ -23,31 +23,14 @@
 // the reference to float rounding).
 #include <algorithm>
 
-#include "common.cuh"
+#include "cb_common.cuh"
 #include "kernels.h"
 
 namespace ccpi {
 namespace {
 
-__device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
-__device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }
-// std::min(a, b) as the reference evaluates it: (b < a) ? b : a.  Every
-// call passes b = a ray's exit alpha, which is never NaN and never -0, and
-// for such b the NaN-propagating hardware minimum returns the same value for
-// every a (NaN a gives NaN, +-0 a with b > 0 gives a), in one instruction
-// instead of a compare and a select.
-#ifndef CB_FMIN_NAN
-#define CB_FMIN_NAN 1
-#endif
-__device__ __forceinline__ float fmin_ref(float a, float b) {
-#if CB_FMIN_NAN
-  float r;
-  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-#else
-  return (b < a) ? b : a;
-#endif
-}
+__device__ __forceinline__ double dmax(double a, double b) { return cb_dmax(a, b); }
+__device__ __forceinline__ double dmin(double a, double b) { return cb_dmin(a, b); }
 
 // xy walk of ray p1 -> p2 over the whole volume; writes alphas[0..n-1] and
 // cells[0..n-2] (x*ny + y, or -1) with lane 0; returns n (0 if missed).
@@ -190,10 +173,6 @@ constexpr int kFpWarps = 4;
 #ifndef CB_FP_PACKED
 #define CB_FP_PACKED 1
 #endif
-
-// Floats of the slice-plane table copy at the start of the forward
-// projector's shared memory (nz + 1 entries, rounded up to 4).
-__host__ __device__ inline int cb_vz_floats(int nz) { return (nz + 1 + 3) & ~3; }
 
 // Row regimes of a walked ray (c2D.cpp:45-99), evaluated warp-parallel:
 // cells [1, ncom) have every row's slice and its neighbour inside the
@@ -678,56 +657,6 @@ __global__ void __launch_bounds__(kFpWarps * 32, 8)
 }
 
 // ---- backward
-constexpr int kBpThreads = 256;
-constexpr int kBpAngleChunk = 64;
-constexpr int kBpMaxRaysPerAngle = 24;
-
-// Rays (angle a, columns h) crossing voxel column [x0,xn) x [y0,yn), with
-// their entry/exit alphas (bproject_ah, c2D.cpp:831-936).  Calls f(h, a0, a1).
-template <class F>
-__device__ void cb_column_rays(const Geom &g, int a, double x0, double xn, double y0,
-                               double yn, F &&f) {
-  const double eps = double(kEps);
-  const double c = g.cosA[a], s = g.sinA[a];
-  const double p1x = g.p1x[a], p1y = g.p1y[a];
-  const double dx0 = x0 - p1x, dy0 = y0 - p1y, dxn = xn - p1x, dyn = yn - p1y;
-  const double cx0 = c * x0 - g.src[0], cxn = c * xn - g.src[0];
-  const double sy0 = s * y0, syn = s * yn;
-  double y00, y01, y10, y11;
-  if (fabs(s) > fabs(c)) {
-    const double il = g.cl / s;
-    y00 = (c - dx0 / (sy0 + cx0)) * il;
-    y01 = (c - dx0 / (syn + cx0)) * il;
-    y10 = (c - dxn / (sy0 + cxn)) * il;
-    y11 = (c - dxn / (syn + cxn)) * il;
-  } else {
-    const double il = g.cl / c;
-    y00 = (-s + dy0 / (cx0 + sy0)) * il;
-    y01 = (-s + dyn / (cx0 + syn)) * il;
-    y10 = (-s + dy0 / (cxn + sy0)) * il;
-    y11 = (-s + dyn / (cxn + syn)) * il;
-  }
-  const int h00 = int(floor(y00 * g.cipix + g.chpix0));
-  const int h01 = int(floor(y01 * g.cipix + g.chpix0));
-  const int h10 = int(floor(y10 * g.cipix + g.chpix0));
-  const int h11 = int(floor(y11 * g.cipix + g.chpix0));
-  const int hmin = max(min(min(h00, h01), min(h10, h11)), 0);
-  const int hmax = min(max(max(h00, h01), max(h10, h11)), g.nh - 1);
-  for (int h = hmin; h <= hmax; h++) {
-    const double p2x = g.cdx[a] - s * g.hpix[h];
-    const double p2y = g.sdx[a] + c * g.hpix[h];
-    const double ddx = p2x - p1x, ddy = p2y - p1y;
-    if (fabs(ddx) < eps || fabs(ddy) < eps)
-      continue; // rejected by the reference ("Ooops", c2D.cpp:909-912)
-    const double idx = 1.0 / ddx, idy = 1.0 / ddy;
-    const double ax0 = dx0 * idx, ay0 = dy0 * idy, axn = dxn * idx, ayn = dyn * idy;
-    const double amin = dmax(dmax(dmin(ax0, axn), dmin(ay0, ayn)), 0.0);
-    const double amax = dmin(dmin(dmax(ax0, axn), dmax(ay0, ayn)), 1.0);
-    if (amin < amax - eps)
-      f(h, float(amin), float(amax));
-  }
-}
-
 // Band rows [lo, hi) of a ray entering a column at a0: rows whose slice and
 // its neighbour stay inside the column (c2D.cpp:664-668).
 __device__ __forceinline__ int cb_band_lo(const Geom &g, float a0) {
@@ -760,580 +689,6 @@ __global__ void __launch_bounds__(kBandWarps * 32) cb_column_band_kernel(Geom g,
   hi = __reduce_min_sync(0xffffffffu, hi);
   if (lane == 0)
     band[col] = make_int2(lo, hi);
-}
-
-template <int EPI>
-__global__ void __launch_bounds__(kBpThreads)
-    cb_bp_kernel(Geom g, const float *__restrict__ pix, float *__restrict__ vol, Epi e,
-                 int *err) {
-  extern __shared__ unsigned char smem_raw[];
-  float *acc = reinterpret_cast<float *>(smem_raw);
-  const int cap = kBpAngleChunk * kBpMaxRaysPerAngle;
-  int *seg_ah = reinterpret_cast<int *>(acc + g.nz);
-  float *seg_a0 = reinterpret_cast<float *>(seg_ah + cap);
-  float *seg_a1 = seg_a0 + cap;
-  __shared__ int s_count, s_minv, s_maxv, s_ovf;
-  const int col = blockIdx.x;
-  const int i = col / g.ny, j = col - (col / g.ny) * g.ny;
-  const double x0 = g.origin[0] + double(i) * g.size[0];
-  const double xn = g.origin[0] + double(i + 1) * g.size[0];
-  const double y0 = g.origin[1] + double(j) * g.size[1];
-  const double yn = g.origin[1] + double(j + 1) * g.size[1];
-  for (int z = threadIdx.x; z < g.nz; z += blockDim.x)
-    acc[z] = 0.0f;
-  if (threadIdx.x == 0) {
-    // rows [min_v, max_v) stay inside the column for every ray
-    // (c2D.cpp:657-676), from the plan's table
-    const int2 b = g.colband[col];
-    s_minv = b.x;
-    s_maxv = b.y;
-    s_ovf = 0;
-  }
-  __syncthreads();
-  const int min_v = s_minv, max_v = s_maxv;
-  const int nzm1 = g.nz - 1, mid = g.mid;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  for (int ac = 0; ac < g.na; ac += kBpAngleChunk) {
-    if (threadIdx.x == 0)
-      s_count = 0;
-    __syncthreads();
-    for (int a = ac + threadIdx.x; a < min(g.na, ac + kBpAngleChunk); a += blockDim.x) {
-      cb_column_rays(g, a, x0, xn, y0, yn, [&](int h, float a0, float a1) {
-        const int slot = atomicAdd(&s_count, 1);
-        if (slot < cap) {
-          seg_ah[slot] = a * g.nh + h;
-          seg_a0[slot] = a0;
-          seg_a1[slot] = a1;
-        } else {
-          s_ovf = 1;
-        }
-      });
-    }
-    __syncthreads();
-    const int nseg = min(s_count, cap);
-    for (int sgi = wib; sgi < nseg; sgi += kBpThreads / 32) {
-      const int ah = seg_ah[sgi];
-      const int h = ah % g.nh;
-      const float a0 = seg_a0[sgi], a1 = seg_a1[sgi];
-      const float av = __fmul_rn(a0, g.inv_dz);
-      const float *prow = pix + i64(ah) * g.nv;
-      const float *drow = g.dconv + i64(h) * g.nv;
-      for (int v = lane; v < g.nv; v += 32) {
-        const float p = __fmul_rn(__ldg(prow + v), __ldg(drow + v));
-        const float dzv = g.dz[v], izv = g.iz[v];
-        if (v >= min_v && v < max_v) {
-          const int k = int(__fadd_rn(g.pzbz, __fmul_rn(av, dzv)));
-          if (v < mid) {
-            if (k < 1 || k > nzm1)
-              continue;
-            const float mz = fmin_ref(__fmul_rn(g.vz[k], izv), a1);
-            atomicAdd(acc + k, __fmul_rn(p, __fsub_rn(mz, a0)));
-            atomicAdd(acc + k - 1, __fmul_rn(p, __fsub_rn(a1, mz)));
-          } else {
-            if (k < 0 || k >= nzm1)
-              continue;
-            const float mz = fmin_ref(__fmul_rn(g.vz[k + 1], izv), a1);
-            atomicAdd(acc + k, __fmul_rn(p, __fsub_rn(mz, a0)));
-            atomicAdd(acc + k + 1, __fmul_rn(p, __fsub_rn(a1, mz)));
-          }
-        } else if (v < min_v) {
-          const int k = int(__fadd_rn(g.pzbz1, __fmul_rn(av, dzv))) - 1;
-          if (k > 0 && k <= nzm1) {
-            const float mz = fmin_ref(__fmul_rn(g.vz[k], izv), a1);
-            atomicAdd(acc + k, __fmul_rn(p, __fsub_rn(mz, a0)));
-            atomicAdd(acc + k - 1, __fmul_rn(p, __fsub_rn(a1, mz)));
-          } else if (k == 0) {
-            const float mz = fmin_ref(__fmul_rn(g.vz[0], izv), a1);
-            atomicAdd(acc, __fmul_rn(p, __fsub_rn(mz, a0)));
-          }
-        } else {
-          const int k = int(__fadd_rn(g.pzbz, __fmul_rn(av, dzv)));
-          if (k < nzm1 && k >= 0) {
-            const float mz = fmin_ref(__fmul_rn(g.vz[k + 1], izv), a1);
-            atomicAdd(acc + k, __fmul_rn(p, __fsub_rn(mz, a0)));
-            atomicAdd(acc + k + 1, __fmul_rn(p, __fsub_rn(a1, mz)));
-          } else if (k == nzm1) {
-            const float mz = fmin_ref(__fmul_rn(g.vz[k + 1], izv), a1);
-            atomicAdd(acc + k, __fmul_rn(p, __fsub_rn(mz, a0)));
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0 && s_ovf)
-    atomicExch(err, 2);
-  double ssq = 0.0;
-  const i64 base = i64(col) * g.nz;
-  for (int z = threadIdx.x; z < g.nz; z += blockDim.x) {
-    const float v = acc[z];
-    float o = v;
-    if (EPI == EPI_NORM) {
-      ssq += double(v) * double(v);
-    } else if (EPI == EPI_SIRT) {
-      const float t = __fadd_rn(e.x[base + z], __fmul_rn(1.0f, __fmul_rn(v, e.w[base + z])));
-      o = (t < 0.0f) ? 0.0f : t;
-    } else if (EPI == EPI_MLEM) {
-      const float t = __fmul_rn(e.x[base + z], __fmul_rn(e.w[base + z], v));
-      o = (t < 0.0f) ? 0.0f : t;
-    }
-    vol[base + z] = o;
-  }
-  if (EPI == EPI_NORM) {
-    __shared__ double red[kBpThreads / 32];
-    const double t = cta_sum<kBpThreads / 32>(ssq, red);
-    if (threadIdx.x == 0)
-      e.partials[blockIdx.x] = t;
-  }
-}
-
-// ---- backward, deterministic gather in the reference's summation order
-//
-// cone_beam::calc_ah_z (c2D.cpp:640-751) adds, for every voxel of a column,
-// first the band rows of every ray (list order: angle, then detector
-// column; rows ascending, each row feeding its slice k and the neighbour
-// k -/+ 1), then the edge rows of every ray (below the band descending,
-// above it ascending).  Here one CTA owns one column and each thread owns
-// NZT of its voxels.  Rays are staged per angle chunk.  For a stage of
-// kGaStage rays each thread loads its band rows (RMAX per ray, all loads in
-// flight together), forms every row's two contributions exactly as the
-// reference does (p (mz - a0) for the row's slice k, p (a1 - mz) for its
-// neighbour) and records, for every slice K, the first band row whose index
-// reaches K (k is monotone in the row).  Each voxel thread then adds, per
-// ray, exactly the contributions that go to its voxel, in the reference's
-// order, so every voxel's sum is formed in the same order with the same
-// unfused float operations as the reference.
-constexpr int kGaThreads = 256;
-constexpr int kGaChunk = 64;
-constexpr int kGaRays = kBpMaxRaysPerAngle; // slots per angle
-#ifndef CB_GA_STAGE
-#define CB_GA_STAGE 3 // rays per stage when the kernel multiplies by d_conv itself
-#endif
-#ifndef CB_GA_STAGE_PRE
-#define CB_GA_STAGE_PRE 4 // rays per stage on a sinogram already scaled by d_conv
-#endif
-#ifndef CB_GA_FAST
-#define CB_GA_FAST 1
-#endif
-#ifndef CB_GA_PACKED
-#define CB_GA_PACKED 1
-#endif
-#ifndef CB_GA_TILE
-#define CB_GA_TILE 16 // CTAs walk the columns in 16 x 16 tiles (0: row-major order)
-#endif
-constexpr int kGaStageMax = 8;
-
-__host__ __device__ inline int round4(int n) { return (n + 3) & ~3; }
-
-// Shared-memory layout of cb_bp_gather (offsets in 4-byte words) for
-// `st` rays per stage.
-struct GaLayout {
-  int vz, dz, iz, seg_h, seg_a0, seg_a1, cnt, off, map, fr, prow, drow, total;
-  __host__ __device__ GaLayout(int nz, int nv, int st) {
-    vz = 0;
-    dz = vz + cb_vz_floats(nz);
-    iz = dz + round4(nv);
-    seg_h = iz + round4(nv);
-    seg_a0 = seg_h + kGaChunk * kGaRays;
-    seg_a1 = seg_a0 + kGaChunk * kGaRays;
-    cnt = seg_a1 + kGaChunk * kGaRays;
-    off = cnt + round4(kGaChunk + 1);
-    map = off + round4(kGaChunk + 1);
-    fr = map + kGaChunk * kGaRays;
-    prow = fr + st * round4(nz + 2);
-    drow = prow + st * round4(nv);
-    total = drow + st * round4(nv);
-  }
-};
-
-// Voxel column of CTA b: CTAs run through the xy plane in T x T tiles, so
-// the columns in flight at any time form a compact patch whose rays (and
-// the sinogram rows they read) overlap and stay in L2.  Any order gives the
-// same sums: each CTA owns its column.
-__device__ __forceinline__ int cb_ga_column(int b, int nx, int ny) {
-#if CB_GA_TILE > 0
-  constexpr int T = CB_GA_TILE;
-  if (nx % T != 0 || ny % T != 0)
-    return b;
-  const int tile = b / (T * T), in = b - tile * (T * T);
-  const int tpr = ny / T; // tiles along y
-  const int ti = tile / tpr, tj = tile - ti * tpr;
-  return (ti * T + in / T) * ny + tj * T + in % T;
-#else
-  return b;
-#endif
-}
-
-// Stage the rays of angles [ac, ac + nac) in list order: slots per angle,
-// then a prefix over angles and a flat map.  Returns the ray count.  Each
-// slot holds the ray's detector column h and its entry and exit alphas.
-__device__ int cb_ga_stage_rays(const Geom &g, int ac, int nac, double x0, double xn, double y0,
-                                double yn, int *seg_h, float *seg_a0, float *seg_a1, int *cnt,
-                                int *off, int *map, int *ovf) {
-  const int tid = threadIdx.x;
-  if (tid < nac) {
-    int c = 0;
-    cb_column_rays(g, ac + tid, x0, xn, y0, yn, [&](int h, float a0, float a1) {
-      if (c < kGaRays) {
-        const int idx = tid * kGaRays + c;
-        seg_h[idx] = h;
-        seg_a0[idx] = a0;
-        seg_a1[idx] = a1;
-      }
-      c++;
-    });
-    if (c > kGaRays) {
-      *ovf = 1;
-      c = kGaRays;
-    }
-    cnt[tid] = c;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int acc = 0;
-    for (int t = 0; t < nac; t++) {
-      off[t] = acc;
-      acc += cnt[t];
-    }
-    off[nac] = acc;
-  }
-  __syncthreads();
-  if (tid < nac)
-    for (int c = 0; c < cnt[tid]; c++)
-      map[off[tid] + c] = tid * kGaRays + c;
-  __syncthreads();
-  return off[nac];
-}
-
-// First-row table: row v of slice k follows row v - 1 of slice kp, so v is
-// the first band row of the slices kp + 1 .. k (entries 0 .. nz + 1 kept).
-__device__ __forceinline__ void cb_ga_mark(int *f, int kp, int k, int v, int nz) {
-#if CB_GA_FAST
-  if (k == kp + 1 && k >= 0 && k <= nz + 1) {
-    f[k] = v; // the usual step: one slice per row change
-    return;
-  }
-#endif
-  for (int K = max(kp + 1, 0); K <= min(k, nz + 1); K++)
-    f[K] = v;
-}
-
-// Register bound: 4 CTAs per SM for one voxel per thread; taller columns
-// need more shared memory per CTA, which allows 3 (or 2) anyway.
-// PRE: the sinogram is already scaled by d_conv (the reference's dpixels,
-// c2D.cpp:1096-1117, formed by the producer of the back projector's input),
-// so a staged row is one load and no multiply.  ST rays per stage.
-// BATCH: nbatch sinograms (EPI_STORE only); without it the item loop runs
-// once and compiles away.
-template <int EPI, int NZT, int RMAX, bool PRE, int ST, bool BATCH>
-__global__ void __launch_bounds__(kGaThreads, NZT == 1 ? 4 : (NZT == 2 ? 3 : 2))
-    cb_bp_gather(Geom g, const float *__restrict__ pix0, float *__restrict__ vol0, Epi e,
-                 int *err, int nbatch) {
-  static_assert(ST <= kGaStageMax, "stage too large");
-  extern __shared__ unsigned char smem_raw[];
-  int *W = reinterpret_cast<int *>(smem_raw);
-  const int nz = g.nz, nv = g.nv, nzm1 = nz - 1, mid = g.mid;
-  const GaLayout L(nz, nv, ST);
-  float *svz = reinterpret_cast<float *>(W + L.vz);
-  float *sdz = reinterpret_cast<float *>(W + L.dz);
-  float *siz = reinterpret_cast<float *>(W + L.iz);
-  int *seg_h = W + L.seg_h;
-  float *seg_a0 = reinterpret_cast<float *>(W + L.seg_a0);
-  float *seg_a1 = reinterpret_cast<float *>(W + L.seg_a1);
-  int *cnt = W + L.cnt, *off = W + L.off, *map = W + L.map, *fr = W + L.fr;
-  float *prow = reinterpret_cast<float *>(W + L.prow); // staged pixel rows
-  float *drow = reinterpret_cast<float *>(W + L.drow); // their d_conv rows
-  const int frs = round4(nz + 2), prs = round4(nv);
-  __shared__ int s_minv, s_maxv, s_ovf;
-  __shared__ int s_kf[ST], s_kl[ST]; // slices of a staged ray's first/last band row
-  // the column's square; kept in shared memory so that its FP64 corners
-  // hold no registers through the row and voxel phases
-  __shared__ double s_box[4];
-  const int tid = threadIdx.x;
-  const int col = cb_ga_column(blockIdx.x, g.nx, g.ny);
-  const int i = col / g.ny, j = col - (col / g.ny) * g.ny;
-  for (int t = tid; t <= nz; t += blockDim.x)
-    svz[t] = g.vz[t];
-  for (int t = tid; t < nv; t += blockDim.x) {
-    sdz[t] = g.dz[t];
-    siz[t] = g.iz[t];
-  }
-  if (tid == 0) {
-    // band limits over every ray of the column (c2D.cpp:657-676), from
-    // the plan's table
-    const int2 b = g.colband[col];
-    s_minv = b.x;
-    s_maxv = b.y;
-    s_ovf = 0;
-    s_box[0] = g.origin[0] + double(i) * g.size[0];
-    s_box[1] = g.origin[0] + double(i + 1) * g.size[0];
-    s_box[2] = g.origin[1] + double(j) * g.size[1];
-    s_box[3] = g.origin[1] + double(j + 1) * g.size[1];
-  }
-  __syncthreads();
-  const int min_v = s_minv, max_v = s_maxv;
-  const int nb = max_v - min_v;
-  const int lo_end = min(mid, max_v);         // lower band rows [min_v, lo_end)
-  const int up_begin = max(mid, min_v);       // upper band rows [up_begin, max_v)
-  const float pzbz = g.pzbz, pzbz1 = g.pzbz1, inv_dz = g.inv_dz;
-  // this thread's band rows v = min_v + tid + r * 256 are the same for every
-  // ray: their z tables stay in registers (sd: delta_z of v, sp: of v - 1,
-  // si: inv_delz of v)
-  float rsd[RMAX], rsp[RMAX], rsi[RMAX];
-#pragma unroll
-  for (int r = 0; r < RMAX; r++) {
-    const int v = min_v + tid + r * kGaThreads;
-    const bool in = v < max_v;
-    rsd[r] = in ? sdz[v] : 0.0f;
-    rsp[r] = (in && v > min_v) ? sdz[v - 1] : 0.0f;
-    rsi[r] = in ? siz[v] : 0.0f;
-  }
-  const float sd_first = nb > 0 ? sdz[min_v] : 0.0f, sd_last = nb > 0 ? sdz[max_v - 1] : 0.0f;
-  double ssq = 0.0;
-  // nbatch sinograms (one after another) share the column's band limits
-  for (int bi = 0; bi < (BATCH ? nbatch : 1); bi++) {
-  const float *__restrict__ pix = pix0 + i64(bi) * g.na * g.nh * nv;
-  float *__restrict__ vol = vol0 + i64(bi) * g.nx * g.ny * nz;
-  float acc[NZT];
-#pragma unroll
-  for (int q = 0; q < NZT; q++)
-    acc[q] = 0.0f;
-
-  // ---- band rows of every ray (c2D.cpp:680-713)
-  for (int ac = 0; nb > 0 && ac < g.na; ac += kGaChunk) {
-    const int nac = min(kGaChunk, g.na - ac);
-    const int nseg = cb_ga_stage_rays(g, ac, nac, s_box[0], s_box[1], s_box[2], s_box[3], seg_h,
-                                      seg_a0, seg_a1, cnt, off, map, &s_ovf);
-    for (int s0 = 0; s0 < nseg; s0 += ST) {
-      const int ns = min(ST, nseg - s0);
-      // 1) this thread's band rows v = min_v + tid + r * 256 of every staged
-      //    ray: pixel values (times d_conv unless pre-scaled), all loads
-      //    issued together
-      float pv[ST][RMAX], dv[PRE ? 1 : ST][RMAX];
-#pragma unroll
-      for (int s = 0; s < ST; s++) {
-        const int m = map[s0 + (s < ns ? s : 0)];
-        const int h = seg_h[m];
-        const float *prw = pix + (i64(ac + m / kGaRays) * g.nh + h) * nv;
-#pragma unroll
-        for (int r = 0; r < RMAX; r++) {
-          const int v = min_v + tid + r * kGaThreads;
-          const bool ok = s < ns && v < max_v;
-          pv[s][r] = ok ? __ldg(prw + v) : 0.0f;
-        }
-        if (!PRE) {
-          const float *drw = g.dconv + i64(h) * nv;
-#pragma unroll
-          for (int r = 0; r < RMAX; r++) {
-            const int v = min_v + tid + r * kGaThreads;
-            dv[PRE ? 0 : s][r] = (s < ns && v < max_v) ? __ldg(drw + v) : 0.0f;
-          }
-        }
-      }
-      // 2) per ray: the first band row of every slice index (the whole
-      //    table: below the first row's slice min_v, above the last row's
-      //    max_v) and each row's two contributions as the reference forms
-      //    them (c2D.cpp:694-711): c1 = p (mz - a0) goes to slice k, c2 =
-      //    p (a1 - mz) to k - 1 below the source row, to k + 1 from it on
-#pragma unroll
-      for (int s = 0; s < ST; s++) {
-        if (s >= ns)
-          break;
-        const int m = map[s0 + s];
-        const float a0 = seg_a0[m], a1 = seg_a1[m];
-        const float av = __fmul_rn(a0, inv_dz);
-        int *f = fr + s * frs;
-        const int kf = int(__fadd_rn(pzbz, __fmul_rn(av, sd_first)));
-        const int kl = int(__fadd_rn(pzbz, __fmul_rn(av, sd_last)));
-#if CB_GA_FAST
-        // only voxels kf - 1 .. kl + 1 receive rows of this ray, and they
-        // read entries kf - 2 .. kl + 3: the band rows' transitions write
-        // (kf, kl], six threads write the ends
-        if (tid < 6) {
-          const int K = tid < 3 ? kf - tid : kl + tid - 2;
-          if (K >= 0 && K <= nz + 1)
-            f[K] = tid < 3 ? min_v : max_v;
-        }
-        if (tid == 0) {
-          s_kf[s] = kf;
-          s_kl[s] = kl;
-        }
-#else
-        for (int K = tid; K <= nz + 1; K += kGaThreads) {
-          if (K <= kf)
-            f[K] = min_v;
-          else if (K > kl)
-            f[K] = max_v;
-        }
-#endif
-        float *c1 = prow + s * prs, *c2 = drow + s * prs;
-#if CB_GA_PACKED
-        const float2 av2 = make_float2(av, av), a02 = make_float2(a0, a0),
-                     a12 = make_float2(a1, a1);
-#endif
-#pragma unroll
-        for (int r = 0; r < RMAX; r++) {
-#if CB_GA_PACKED
-          if (r + 1 < RMAX && (r & 1) == 0) {
-            // rows r and r + 1 as packed pairs: the same unfused float
-            // operations per row, two rows per multiply and subtract
-            const int v0 = min_v + tid + r * kGaThreads, v1 = v0 + kGaThreads;
-            const float2 kk = mul2_rn(av2, make_float2(rsd[r], rsd[r + 1]));
-            const float2 kq = mul2_rn(av2, make_float2(rsp[r], rsp[r + 1]));
-            const int k0 = int(__fadd_rn(pzbz, kk.x)), k1 = int(__fadd_rn(pzbz, kk.y));
-            if (v0 < max_v && v0 > min_v)
-              cb_ga_mark(f, int(__fadd_rn(pzbz, kq.x)), k0, v0, nz);
-            if (v1 < max_v)
-              cb_ga_mark(f, int(__fadd_rn(pzbz, kq.y)), k1, v1, nz);
-            const int kz0 = min(max(v0 < mid ? k0 : k0 + 1, 0), nz);
-            const int kz1 = min(max(v1 < mid ? k1 : k1 + 1, 0), nz);
-            const float2 pl =
-                mul2_rn(make_float2(svz[kz0], svz[kz1]), make_float2(rsi[r], rsi[r + 1]));
-            const float2 mz = make_float2(fmin_ref(pl.x, a1), fmin_ref(pl.y, a1));
-            const float2 p = PRE ? make_float2(pv[s][r], pv[s][r + 1])
-                                 : mul2_rn(make_float2(pv[s][r], pv[s][r + 1]),
-                                           make_float2(dv[PRE ? 0 : s][r], dv[PRE ? 0 : s][r + 1]));
-            const float2 w1 = mul2_rn(p, sub2_rn(mz, a02)), w2 = mul2_rn(p, sub2_rn(a12, mz));
-            if (v0 < max_v) {
-              c1[v0] = w1.x;
-              c2[v0] = w2.x;
-            }
-            if (v1 < max_v) {
-              c1[v1] = w1.y;
-              c2[v1] = w2.y;
-            }
-            continue;
-          }
-          if (r & 1)
-            continue; // done with its pair
-#endif
-          const int v = min_v + tid + r * kGaThreads;
-          if (v < max_v) {
-            const int k = int(__fadd_rn(pzbz, __fmul_rn(av, rsd[r])));
-            if (v > min_v)
-              cb_ga_mark(f, int(__fadd_rn(pzbz, __fmul_rn(av, rsp[r]))), k, v, nz);
-            const int kz = min(max(v < mid ? k : k + 1, 0), nz);
-            const float mz = fmin_ref(__fmul_rn(svz[kz], rsi[r]), a1);
-            const float p = PRE ? pv[s][r] : __fmul_rn(pv[s][r], dv[PRE ? 0 : s][r]);
-            c1[v] = __fmul_rn(p, __fsub_rn(mz, a0));
-            c2[v] = __fmul_rn(p, __fsub_rn(a1, mz));
-          }
-        }
-      }
-      __syncthreads();
-      // 3) each voxel adds its rows' contributions in the reference's order
-      for (int s = 0; s < ns; s++) {
-        const int *f = fr + s * frs;
-        const float *c1 = prow + s * prs, *c2 = drow + s * prs;
-#if CB_GA_FAST
-        const int klo = s_kf[s] - 1, khi = s_kl[s] + 1;
-#endif
-#pragma unroll
-        for (int q = 0; q < NZT; q++) {
-          const int K = tid + q * kGaThreads;
-          if (K >= nz)
-            continue;
-#if CB_GA_FAST
-          if (K < klo || K > khi)
-            continue; // no row of this ray feeds voxel K
-#endif
-          const int fm = K >= 1 ? f[K - 1] : min_v, f0 = f[K], f1 = f[K + 1];
-          float t = acc[q];
-          // below the source row: rows of slice K give c1, then rows of
-          // slice K + 1 give c2 (their neighbour k - 1 == K)
-          for (int v = f0, ve = min(f[K + 2], lo_end); v < ve; v++)
-            t = __fadd_rn(t, (v < f1 ? c1 : c2)[v]);
-          // from the source row on: rows of slice K - 1 give c2 (their
-          // neighbour k + 1 == K), then rows of slice K give c1
-          for (int v = max(fm, up_begin), ve = min(f1, max_v); v < ve; v++)
-            t = __fadd_rn(t, (v < f0 ? c2 : c1)[v]);
-          acc[q] = t;
-        }
-      }
-      __syncthreads();
-    }
-  }
-
-  // ---- edge rows of every ray (c2D.cpp:715-750)
-  if (min_v > 0 || max_v < nv) {
-    for (int ac = 0; ac < g.na; ac += kGaChunk) {
-      const int nac = min(kGaChunk, g.na - ac);
-      const int nseg = cb_ga_stage_rays(g, ac, nac, s_box[0], s_box[1], s_box[2], s_box[3],
-                                        seg_h, seg_a0, seg_a1, cnt, off, map, &s_ovf);
-      for (int s = 0; s < nseg; s++) {
-        const int m = map[s];
-        const int h = seg_h[m];
-        const float a0 = seg_a0[m], a1 = seg_a1[m];
-        const float av = __fmul_rn(a0, inv_dz);
-        const float *prw = pix + (i64(ac + m / kGaRays) * g.nh + h) * nv;
-        const float *drw = g.dconv + i64(h) * nv;
-#pragma unroll
-        for (int q = 0; q < NZT; q++) {
-          const int K = tid + q * kGaThreads;
-          if (K >= nz)
-            continue;
-          for (int v = min(min_v, nv) - 1; v >= 0; v--) {
-            const int k = int(__fadd_rn(pzbz1, __fmul_rn(av, sdz[v]))) - 1;
-            if (k < K)
-              break; // k only falls as v falls (and k < 0 ends the reference's loop)
-            if (k > K + 1)
-              continue;
-            const float p = PRE ? __ldg(prw + v) : __fmul_rn(__ldg(prw + v), __ldg(drw + v));
-            if (k > 0) {
-              const float mz = fmin_ref(__fmul_rn(svz[k], siz[v]), a1);
-              acc[q] = __fadd_rn(acc[q], __fmul_rn(p, k == K ? __fsub_rn(mz, a0)
-                                                             : __fsub_rn(a1, mz)));
-            } else if (K == 0) {
-              const float mz = fmin_ref(__fmul_rn(svz[0], siz[v]), a1);
-              acc[q] = __fadd_rn(acc[q], __fmul_rn(p, __fsub_rn(mz, a0)));
-            }
-          }
-          for (int v = max(max_v, 0); v < nv; v++) {
-            const int k = int(__fadd_rn(pzbz, __fmul_rn(av, sdz[v])));
-            if (k > K || k > nzm1)
-              break; // k only rises with v (and k > nz - 1 ends the reference's loop)
-            if (k < K - 1)
-              continue;
-            const float p = PRE ? __ldg(prw + v) : __fmul_rn(__ldg(prw + v), __ldg(drw + v));
-            const float mz = fmin_ref(__fmul_rn(svz[k + 1], siz[v]), a1);
-            if (k == K)
-              acc[q] = __fadd_rn(acc[q], __fmul_rn(p, __fsub_rn(mz, a0)));
-            else if (k < nzm1)
-              acc[q] = __fadd_rn(acc[q], __fmul_rn(p, __fsub_rn(a1, mz)));
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  const i64 base = i64(col) * nz;
-#pragma unroll
-  for (int q = 0; q < NZT; q++) {
-    const int K = tid + q * kGaThreads;
-    if (K >= nz)
-      continue;
-    const float v = acc[q];
-    float o = v;
-    if (EPI == EPI_NORM) {
-      ssq += double(v) * double(v);
-    } else if (EPI == EPI_SIRT) {
-      const float t = __fadd_rn(e.x[base + K], __fmul_rn(1.0f, __fmul_rn(v, e.w[base + K])));
-      o = (t < 0.0f) ? 0.0f : t;
-    } else if (EPI == EPI_MLEM) {
-      const float t = __fmul_rn(e.x[base + K], __fmul_rn(e.w[base + K], v));
-      o = (t < 0.0f) ? 0.0f : t;
-    }
-    vol[base + K] = o;
-  }
-  } // batch items
-  if (tid == 0 && s_ovf)
-    atomicExch(err, 2);
-  if (EPI == EPI_NORM) {
-    __shared__ double red[kGaThreads / 32];
-    const double t = cta_sum<kGaThreads / 32>(ssq, red);
-    if (threadIdx.x == 0)
-      e.partials[blockIdx.x] = t;
-  }
 }
 
 } // namespace
@@ -1438,33 +793,9 @@ void launch_cb_fp(const Geom &g, const float *vol, float *pix, const Epi &e, con
 }
 } // namespace
 
-namespace {
-size_t cb_bp_atomic_smem(const Geom &g) {
-  return size_t(g.nz) * sizeof(float) +
-         size_t(kBpAngleChunk) * kBpMaxRaysPerAngle * (sizeof(int) + 2 * sizeof(float));
-}
-// the larger of the two stage sizes' layouts
-size_t cb_bp_gather_smem(const Geom &g) {
-  return size_t(GaLayout(g.nz, g.nv, std::max(CB_GA_STAGE, CB_GA_STAGE_PRE)).total) * 4;
-}
-// voxels per thread of the deterministic gather, 0 if it does not apply
-int cb_bp_gather_nzt(const Geom &g) {
-  if (cb_bp_gather_smem(g) > 200 * 1024 || g.nv > 4 * kGaThreads)
-    return 0;
-  return g.nz <= kGaThreads ? 1 : g.nz <= 2 * kGaThreads ? 2 : g.nz <= 4 * kGaThreads ? 4 : 0;
-}
-// band rows per thread of the deterministic gather (nv <= 1024)
-int cb_bp_gather_rmax(const Geom &g) { return (g.nv + kGaThreads - 1) / kGaThreads; }
-} // namespace
-
-size_t cb_bp_smem(const Geom &g) {
-  return cb_bp_gather_nzt(g) ? cb_bp_gather_smem(g) : cb_bp_atomic_smem(g);
-}
-
-int cb_prepare(const Geom &g) {
-  const int fp = int(cb_fp_smem(g)), bp = int(cb_bp_atomic_smem(g));
-  const int ga = int(cb_bp_gather_smem(g));
-  cudaError_t e1 = cudaSuccess, e2 = cudaSuccess;
+int cb_prepare() {
+  // the limit is the function's, not the plan's: the largest any plan uses
+  const int fp = 200 * 1024;
 #define CB_FP_ALL(R, F)                                                                    \
   (const void *)cb_fp_kernel<EPI_STORE, R, F, false>,                                       \
       (const void *)cb_fp_kernel<EPI_NORM, R, F, false>,                                    \
@@ -1480,35 +811,10 @@ int cb_prepare(const Geom &g) {
                        (const void *)cb_bp_scatter<3, false>,
                        (const void *)cb_bp_scatter<3, true>};
 #undef CB_FP_ALL
-  const void *bps[] = {(const void *)cb_bp_kernel<EPI_STORE>, (const void *)cb_bp_kernel<EPI_NORM>,
-                       (const void *)cb_bp_kernel<EPI_SIRT>, (const void *)cb_bp_kernel<EPI_MLEM>};
   for (const void *f : fps)
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, fp) != cudaSuccess)
-      e1 = cudaErrorInvalidValue;
-  for (const void *f : bps)
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bp) != cudaSuccess)
-      e2 = cudaErrorInvalidValue;
-  if (cb_bp_gather_nzt(g)) {
-#define CB_GA_EPI(Z, R)                                                                    \
-  (const void *)cb_bp_gather<EPI_STORE, Z, R, false, CB_GA_STAGE, false>,                   \
-      (const void *)cb_bp_gather<EPI_NORM, Z, R, false, CB_GA_STAGE, false>,                \
-      (const void *)cb_bp_gather<EPI_SIRT, Z, R, false, CB_GA_STAGE, false>,                \
-      (const void *)cb_bp_gather<EPI_MLEM, Z, R, false, CB_GA_STAGE, false>,                \
-      (const void *)cb_bp_gather<EPI_STORE, Z, R, true, CB_GA_STAGE_PRE, false>,            \
-      (const void *)cb_bp_gather<EPI_NORM, Z, R, true, CB_GA_STAGE_PRE, false>,             \
-      (const void *)cb_bp_gather<EPI_SIRT, Z, R, true, CB_GA_STAGE_PRE, false>,             \
-      (const void *)cb_bp_gather<EPI_MLEM, Z, R, true, CB_GA_STAGE_PRE, false>,             \
-      (const void *)cb_bp_gather<EPI_STORE, Z, R, false, CB_GA_STAGE, true>,                \
-      (const void *)cb_bp_gather<EPI_STORE, Z, R, true, CB_GA_STAGE_PRE, true>
-#define CB_GA_ALL(Z) CB_GA_EPI(Z, 1), CB_GA_EPI(Z, 2), CB_GA_EPI(Z, 3), CB_GA_EPI(Z, 4)
-    const void *gas[] = {CB_GA_ALL(1), CB_GA_ALL(2), CB_GA_ALL(4)};
-#undef CB_GA_EPI
-#undef CB_GA_ALL
-    for (const void *f : gas)
-      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, ga) != cudaSuccess)
-        e2 = cudaErrorInvalidValue;
-  }
-  return (e1 == cudaSuccess && e2 == cudaSuccess) ? 0 : 1;
+      return 1;
+  return cb_bp_prepare();
 }
 
 int cb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi &e,
@@ -1525,103 +831,6 @@ int cb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi 
     break;
   case EPI_MLEM:
     launch_cb_fp<EPI_MLEM>(g, vol, pix, e, hrange, grid, st, nb);
-    break;
-  default:
-    return 1;
-  }
-  return 0;
-}
-
-namespace {
-// out[a][h][v] = in[a][h][v] * d_conv[h][v]: the reference's dpixels
-// (c2D.cpp:1096-1117), the same float products the back projector would
-// form row by row.
-__global__ void cb_prescale_kernel(const float *__restrict__ in, float *__restrict__ out,
-                                   const float *__restrict__ dconv, i64 per_angle, i64 n) {
-  for (i64 i = blockIdx.x * i64(blockDim.x) + threadIdx.x; i < n;
-       i += i64(gridDim.x) * blockDim.x)
-    out[i] = __fmul_rn(in[i], dconv[i % per_angle]);
-}
-
-template <int EPI, bool PRE, int ST>
-void launch_cb_ga(const Geom &g, int nzt, int rmax, const float *pix, float *vol, const Epi &e,
-                  int *err, cudaStream_t st, int nbatch) {
-  const int ncol = g.nx * g.ny;
-  const size_t gsm = cb_bp_gather_smem(g);
-#define CB_GA_ONE(Z, R, B)                                                                 \
-  cb_bp_gather<EPI, Z, R, PRE, ST, B><<<ncol, kGaThreads, gsm, st>>>(g, pix, vol, e, err, nbatch)
-#define CB_GA_GO(Z, B)                                                                     \
-  (rmax == 1   ? CB_GA_ONE(Z, 1, B)                                                         \
-   : rmax == 2 ? CB_GA_ONE(Z, 2, B)                                                         \
-   : rmax == 3 ? CB_GA_ONE(Z, 3, B)                                                         \
-               : CB_GA_ONE(Z, 4, B))
-  if constexpr (EPI == EPI_STORE) {
-    if (nbatch > 1) {
-      if (nzt == 1)
-        CB_GA_GO(1, true);
-      else if (nzt == 2)
-        CB_GA_GO(2, true);
-      else
-        CB_GA_GO(4, true);
-      return;
-    }
-  }
-  if (nzt == 1)
-    CB_GA_GO(1, false);
-  else if (nzt == 2)
-    CB_GA_GO(2, false);
-  else
-    CB_GA_GO(4, false);
-#undef CB_GA_GO
-#undef CB_GA_ONE
-}
-
-template <int EPI>
-void launch_cb_bp(const Geom &g, const float *pix, float *vol, const Epi &e, int *err,
-                  cudaStream_t st, int nbatch) {
-  const int ncol = g.nx * g.ny;
-  const int nzt = cb_bp_gather_nzt(g), rmax = cb_bp_gather_rmax(g);
-  if (nzt && e.pre) {
-    launch_cb_ga<EPI, true, CB_GA_STAGE_PRE>(g, nzt, rmax, pix, vol, e, err, st, nbatch);
-    return;
-  }
-  switch (nzt) {
-  case 1:
-  case 2:
-  case 4:
-    launch_cb_ga<EPI, false, CB_GA_STAGE>(g, nzt, rmax, pix, vol, e, err, st, nbatch);
-    break;
-  default:
-    // columns taller than the gather handles: one launch per batch item
-    for (int b = 0; b < nbatch; b++)
-      cb_bp_kernel<EPI><<<ncol, kBpThreads, cb_bp_atomic_smem(g), st>>>(
-          g, pix + i64(b) * g.na * g.nh * g.nv, vol + i64(b) * g.nx * g.ny * g.nz, e, err);
-  }
-}
-} // namespace
-
-bool cb_bp_takes_prescaled(const Geom &g) { return cb_bp_gather_nzt(g) != 0; }
-
-void cb_prescale(const Geom &g, const float *in, float *out, cudaStream_t st) {
-  const i64 per = i64(g.nh) * g.nv, n = i64(g.na) * per;
-  const i64 blocks = std::min<i64>((n + 255) / 256, i64(sm_count()) * 8);
-  cb_prescale_kernel<<<int(std::max<i64>(blocks, 1)), 256, 0, st>>>(in, out, g.dconv, per, n);
-}
-
-int cb_backward(const Geom &g, const float *pix, float *vol, int mode, const Epi &e,
-                int *err, cudaStream_t st, int nbatch) {
-  switch (mode) {
-  case EPI_STORE:
-    launch_cb_bp<EPI_STORE>(g, pix, vol, e, err, st, nbatch);
-    break;
-  case EPI_NORM:
-    launch_cb_bp<EPI_NORM>(g, pix, vol, e, err, st, nbatch);
-    break;
-  case EPI_SIRT:
-    launch_cb_bp<EPI_SIRT>(g, pix, vol, e, err, st, nbatch);
-    break;
-  case EPI_MLEM:
-    launch_cb_bp<EPI_MLEM>(g, pix, vol, e, err, st, nbatch);
     break;
   default:
     return 1;

@@ -50,6 +50,11 @@ struct Geom {
   const float *vz;        // nz + 1: slice planes relative to src_z
   float inv_dz, pzbz, pzbz1, pzdv, z1, znm, pzdeps;
   int mid;                // first row above the source
+  float dz0, inv_pitch, pitch_max; // dz[0], 1 / mean row step, largest row step
+  int even_rows;          // every row within a quarter step of dz0 + v / inv_pitch
+  const double2 *inv;     // na * nh: 1 / the ray's x and y spans (x = 0: the back
+                          // projector takes no such ray, c2D.cpp:909-912)
+  float neg0;             // -0.0f (see mul2_nz)
   // nx * ny: per voxel column the back projector's band rows [x, y) that
   // stay inside the column for every ray crossing it (c2D.cpp:657-676)
   const int2 *colband;
@@ -123,6 +128,35 @@ __device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
       "mov.b64 {%0, %1}, z;\n\t}"
       : "=f"(r.x), "=f"(r.y)
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
+__device__ __forceinline__ float2 add2_rz(float2 a, float2 b) {
+  float2 r;
+  asm("{ .reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "add.rz.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
+// a * b as fma(a, b, nz) with nz = -0.0f in both halves: the rounded product
+// (adding -0 changes no value and no sign), which packed adds may take as an
+// operand because ptxas has no multiply left to contract.  nz must reach the
+// kernel as data (Geom::neg0); a literal would be folded away.
+__device__ __forceinline__ float2 mul2_nz(float2 a, float2 b, float2 nz) {
+  float2 r;
+  asm("{ .reg .b64 x, y, z, w;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "mov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 w, x, y, z;\n\t"
+      "mov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(nz.x), "f"(nz.y));
   return r;
 }
 

@@ -260,6 +260,17 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     }
     for (int i = 0; i <= nz; i++)
       vz[i] = float(g.origin[2] + double(i) * g.size[2] - sz);
+    // row spacing: its mean (row estimates) and its largest step (rounded up)
+    g.dz0 = dz[0];
+    g.inv_pitch = float(double(nv - 1) / (double(dz[nv - 1]) - double(dz[0])));
+    g.pitch_max = 0.0f;
+    for (int i = 1; i < nv; i++)
+      g.pitch_max = std::max(g.pitch_max, 1.0001f * (dz[i] - dz[i - 1]));
+    g.even_rows = 1;
+    for (int i = 0; i < nv; i++)
+      if (std::abs((double(dz[i]) - g.dz0) * g.inv_pitch - i) > 0.25)
+        g.even_rows = 0;
+    g.neg0 = -0.0f;
     g.dconv = upload(p, dconv);
     g.dz = upload(p, dz);
     g.iz = upload(p, iz);
@@ -304,24 +315,27 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     p->hrange = upload(p, hr);
     ok = ok && g.p1x && g.p1y && g.cdx && g.sdx && g.dconv && g.dz && g.iz && g.vz &&
          p->hrange;
-    if (cb_fp_smem(g) > 200 * 1024 || cb_bp_smem(g) > 200 * 1024) {
+    if (cb_fp_smem(g) > 200 * 1024 || nz > 46592) {
       set_error("ccpi_plan_create: volume too large for the cone kernels' shared memory");
       delete p;
       return 1;
     }
-    ok = ok && cb_prepare(g) == 0;
+    ok = ok && cb_prepare() == 0;
     if (ok) {
       const std::vector<int2> none(size_t(g.nx) * g.ny, make_int2(0, 0));
       int2 *band = upload(p, none);
-      ok = band && cb_column_bands(g, band, 0) == 0;
+      const std::vector<double2> zero(size_t(na) * nh, make_double2(0.0, 0.0));
+      double2 *inv = upload(p, zero);
+      ok = band && inv && cb_column_bands(g, band, 0) == 0 && cb_ray_spans(g, inv, 0) == 0;
       g.colband = band;
+      g.inv = inv;
     }
     // one CTA per four rays (a warp each) for the forward projector and the
     // scatter: with 8 CTAs per SM looping over the rays, SMs sat idle at the
     // end of a launch (512^3: forward 334 -> 306 ms, scatter 629 -> 518 ms);
     // capped so that the FP64 partial sums stay few on huge ray counts
     p->fp_grid = int(std::min<i64>((i64(na) * nh + 3) / 4, i64(sm_count()) * 1024));
-    p->bp_parts = g.nx * g.ny;
+    p->bp_parts = cb_bp_parts(g);
   }
   void *err = nullptr;
   ok = ok && cudaMalloc(&err, sizeof(int)) == cudaSuccess;
@@ -371,7 +385,7 @@ int set_cone_backprojector(ccpi_plan *p, int scatter) {
   p->g.tune_scatter = scatter ? 1 : 0;
   // one FP64 partial sum per back-projector CTA (gather: one per column),
   // or per block of the sum-of-squares pass after the scatter
-  p->bp_parts = scatter ? sumsq_blocks() : p->g.nx * p->g.ny;
+  p->bp_parts = scatter ? sumsq_blocks() : cb_bp_parts(p->g);
   return 0;
 }
 
@@ -422,7 +436,7 @@ size_t layout(const ccpi_plan *p, int alg, int niter, char *base, Work *w) {
 // first scaled by d_conv into q (free once r is updated), the reference's
 // dpixels, and the back projector reads the scaled copy.
 int backward_residual(const ccpi_plan *p, const Work &W, Epi e, cudaStream_t st) {
-  if (p->g.kind == CCPI_CONE && cb_bp_takes_prescaled(p->g)) {
+  if (p->g.kind == CCPI_CONE) {
     cb_prescale(p->g, W.r, W.q, st);
     e.pre = 1;
     return backward(p, W.q, W.s, EPI_NORM, e, st);
@@ -437,7 +451,7 @@ int iterate(const ccpi_plan *p, int alg, const float *sino, float *x, const Work
   Epi e{};
   // cone SIRT / MLEM: the forward projector stores its residual scaled by
   // d_conv, which the back projector then reads as is
-  const int pre = (p->g.kind == CCPI_CONE && cb_bp_takes_prescaled(p->g)) ? 1 : 0;
+  const int pre = (p->g.kind == CCPI_CONE) ? 1 : 0;
   int rc = 0;
   switch (alg) {
   case CCPI_CGLS:
@@ -1092,7 +1106,7 @@ int plan_autotune(ccpi_plan *p, cudaStream_t st, int *chosen) {
     // form the CGLS iterations run (on a sinogram pre-scaled by d_conv
     // where the gather takes one; the scratch values do not matter)
     Epi pre{};
-    pre.pre = cb_bp_takes_prescaled(p->g) ? 1 : 0;
+    pre.pre = 1;
     const float t_gather = timed([&] {
       cb_backward(p->g, pix, vol, EPI_STORE, pre, p->err, st);
     });

@@ -13,12 +13,14 @@ int pb_fp_ctas(const Geom &g);
 int pb_backward(const Geom &g, const float *pix, float *vol, int mode, const Epi &e,
                 int *err, cudaStream_t st);
 int pb_bp_tiles(const Geom &g);
-int cb_prepare(const Geom &g);
+int cb_prepare();
 // band[i * ny + j] = the back projector's band rows [x, y) of voxel column
 // (i, j) (c2D.cpp:657-676); the cone back projectors read it as g.colband
 int cb_column_bands(const Geom &g, int2 *band, cudaStream_t st);
+// inv[a * nh + h] = the reciprocal x and y spans of every ray as the back
+// projector forms them (Geom::inv)
+int cb_ray_spans(const Geom &g, double2 *inv, cudaStream_t st);
 size_t cb_fp_smem(const Geom &g);
-size_t cb_bp_smem(const Geom &g);
 // nb / nbatch: that many volumes and sinograms one after another, one launch
 // (EPI_STORE); the walk, row regimes and band limits are shared
 int cb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi &e,
@@ -31,9 +33,12 @@ int cb_backward(const Geom &g, const float *pix, float *vol, int mode, const Epi
 // by d_conv.  Launch shape of the forward projector.
 int cb_backward_scatter(const Geom &g, const float *pix, float *vol, int pre,
                         const int2 *hrange, int grid, cudaStream_t st);
-// The cone back projector accepts a sinogram pre-scaled by d_conv (Epi::pre)
-// for this geometry; cb_prescale writes that scaled copy.
-bool cb_bp_takes_prescaled(const Geom &g);
+// CTAs of the cone back projector (= its partial sums); its set-up, done by
+// cb_prepare.
+int cb_bp_parts(const Geom &g);
+int cb_bp_prepare();
+// The cone back projector accepts a sinogram pre-scaled by d_conv
+// (Epi::pre); cb_prescale writes that scaled copy.
 void cb_prescale(const Geom &g, const float *in, float *out, cudaStream_t st);
 // Streaming multiprocessors of the current device (engine.cu).
 int sm_count();
