@@ -29,6 +29,12 @@
 namespace ccpi {
 namespace {
 
+__device__ __forceinline__ float lds_f(unsigned a) {
+  float v;
+  asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+
 __device__ __forceinline__ double dmax(double a, double b) { return cb_dmax(a, b); }
 __device__ __forceinline__ double dmin(double a, double b) { return cb_dmin(a, b); }
 
@@ -170,9 +176,6 @@ __device__ __forceinline__ float cb_fp_epi(float acc, i64 idx, const Epi &e, dou
 }
 
 constexpr int kFpWarps = 4;
-#ifndef CB_FP_PACKED
-#define CB_FP_PACKED 1
-#endif
 
 // Row regimes of a walked ray (c2D.cpp:45-99), evaluated warp-parallel:
 // cells [1, ncom) have every row's slice and its neighbour inside the
@@ -239,15 +242,81 @@ __device__ __forceinline__ void cb_row_regimes(const Geom &g, const float *alpha
   }
 }
 
-// RPL = detector rows per lane per pass (a pass covers 32 * RPL rows);
-// FULL: nv is a multiple of 32 * RPL (no idle rows).  BATCH: nb volumes
-// (one after another) share each ray's walk and row regimes (EPI_STORE
-// only).  Without it the item loop runs once and compiles away: a run-time
-// loop costs the single-volume form 10 % at 512^3.
-template <int EPI, int RPL, bool FULL, bool BATCH>
+// How a pass of 32 * RPL rows lies to the source: all below, all above, or
+// the first half of each lane's rows below and the second above.
+enum Side { BELOW = 0, ABOVE = 1, HALVES = 2 };
+
+// One pass over cells [1, m1), where every row's slice k and the neighbour
+// on the far side of the plane it may cross lie inside the column.  Rows q
+// and q + 1 of a lane go as packed pairs: per row the reference's unfused
+// float operations (c2D.cpp:99-145), in its order.  int(x) is the low bits of
+// 2^23 + x rounded toward zero (1 <= x).  Where the pass lies to the source is
+// a template argument, so the neighbour is an immediate offset.
+//
+// Bound: instruction issue.  Scalar sums and conversions, and the neighbour's
+// address formed per row, took 306 ms at 512^3 / 720 angles / 768^2; packed
+// sums (mul2_nz), int(x) by addition and immediate offsets 260 ms; addresses
+// as multiply-adds by a 4 the compiler cannot turn into shifts, which puts
+// them on the FMA pipe (26 % busy) instead of the ALU (50 %), 232 ms.
+__device__ __forceinline__ const float *at_wide(unsigned k, unsigned four, const char *c) {
+  const float *r;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(k), "r"(four), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned at_smem(unsigned k, unsigned four, unsigned c) {
+  unsigned r;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(k), "r"(four), "r"(c));
+  return r;
+}
+template <int RPL, int SIDE>
+__device__ __forceinline__ void cb_fp_cells(const Geom &g, const float *alphas, const int *cells,
+                                            int m1, const float *vol, const float *svz,
+                                            const float2 (&dz2)[RPL / 2],
+                                            const float2 (&iz2)[RPL / 2],
+                                            float2 (&acc2)[RPL / 2]) {
+  constexpr unsigned kMagic = 0x4b000000u; // bits of 2^23
+  const float2 nz = make_float2(g.neg0, g.neg0);
+  const float2 pz = make_float2(g.pzbz, g.pzbz), big = make_float2(8388608.0f, 8388608.0f);
+  const unsigned vz = unsigned(__cvta_generic_to_shared(svz)) - 4 * kMagic;
+  for (int m = 1; m < m1; m++) {
+    const int cell = cells[m - 1];
+    if (cell < 0)
+      continue;
+    const float a0 = alphas[m - 1], a1 = alphas[m];
+    const char *col = reinterpret_cast<const char *>(vol + i64(cell) * g.nz) - 4ll * kMagic;
+    const float av = __fmul_rn(a0, g.inv_dz);
+    const float2 av2 = make_float2(av, av), a02 = make_float2(a0, a0), a12 = make_float2(a1, a1);
+#pragma unroll
+    for (int q = 0; q < RPL; q += 2) {
+      const float2 x = add2_rn(pz, mul2_nz(av2, dz2[q / 2], nz));
+      const float2 b = add2_rz(x, big);
+      const unsigned k0 = __float_as_uint(b.x), k1 = __float_as_uint(b.y);
+      const int d0 = SIDE == BELOW || (SIDE == HALVES && q < RPL / 2) ? -1 : 1;
+      const int d1 = SIDE == BELOW || (SIDE == HALVES && q + 1 < RPL / 2) ? -1 : 1;
+      const float2 pl = mul2_rn(make_float2(lds_f(at_smem(k0, g.four, vz) + (d0 < 0 ? 0 : 4)),
+                                            lds_f(at_smem(k1, g.four, vz) + (d1 < 0 ? 0 : 4))),
+                                iz2[q / 2]);
+      const float2 mz = make_float2(fmin_ref(pl.x, a1), fmin_ref(pl.y, a1));
+      const float2 lo = sub2_rn(mz, a02), hi = sub2_rn(a12, mz);
+      const float *c0 = at_wide(k0, g.four, col), *c1 = at_wide(k1, g.four, col);
+      const float2 pk = mul2_nz(make_float2(__ldg(c0), __ldg(c1)), lo, nz);
+      const float2 pn = mul2_nz(make_float2(__ldg(c0 + d0), __ldg(c1 + d1)), hi, nz);
+      acc2[q / 2] = add2_rn(acc2[q / 2], add2_rn(pk, pn));
+    }
+  }
+}
+
+// RPL = detector rows per lane per pass.  The np passes of 32 * RPL rows start
+// at row v0 <= 0, such that the first row above the source begins a pass or
+// the second half of one; rows outside [0, nv) act as a row at the source
+// height and are not stored.  BATCH: nb
+// volumes (one after another) share each ray's walk and row regimes
+// (EPI_STORE only).  Without it the item loop runs once and compiles away: a
+// run-time loop costs the single-volume form 10 % at 512^3.
+template <int EPI, int RPL, bool BATCH>
 __global__ void __launch_bounds__(kFpWarps * 32)
     cb_fp_kernel(Geom g, const float *__restrict__ vol0, float *__restrict__ pix0, Epi e,
-                 const int2 *__restrict__ hrange, int cap, int nb) {
+                 const int2 *__restrict__ hrange, int cap, int nb, int v0, int np) {
   extern __shared__ unsigned char smem_raw[];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float *svz = reinterpret_cast<float *>(smem_raw);
@@ -280,14 +349,14 @@ __global__ void __launch_bounds__(kFpWarps * 32)
     // batch item b: its volume and its sinogram
     const float *__restrict__ vol = vol0 + i64(b) * g.nx * g.ny * g.nz;
     float *__restrict__ pix = pix0 + i64(b) * g.na * g.nh * g.nv;
-    for (int vb = 0; vb < g.nv; vb += 32 * RPL) {
+    for (int vb = v0; vb < v0 + np * 32 * RPL; vb += 32 * RPL) {
       float acc[RPL], dzv[RPL], izv[RPL];
       bool vok[RPL], below[RPL];
 #pragma unroll
       for (int q = 0; q < RPL; q++) {
         const int v = vb + q * 32 + lane;
         acc[q] = 0.0f;
-        vok[q] = v < g.nv;
+        vok[q] = v >= 0 && v < g.nv;
         below[q] = v < mid;
         dzv[q] = vok[q] ? g.dz[v] : 0.0f;
         izv[q] = vok[q] ? g.iz[v] : 0.0f;
@@ -295,73 +364,25 @@ __global__ void __launch_bounds__(kFpWarps * 32)
       // In [1, mfast) the regime search has shown that the lowest row's
       // slice index is >= 1 and the highest row's < nz - 1 (c2D.cpp:45-99),
       // so every row's k and its neighbour k -/+ 1 are inside the column.
-      int dk[RPL];
-      const float *vzq[RPL];
+      float2 acc2[RPL / 2], dz2[RPL / 2], iz2[RPL / 2];
 #pragma unroll
-      for (int q = 0; q < RPL; q++) {
-        dk[q] = below[q] ? -1 : 1;
-        vzq[q] = svz + (below[q] ? 0 : 1);
+      for (int q = 0; q < RPL; q += 2) {
+        acc2[q / 2] = make_float2(0.0f, 0.0f);
+        dz2[q / 2] = make_float2(dzv[q], dzv[q + 1]);
+        iz2[q / 2] = make_float2(izv[q], izv[q + 1]);
       }
-#if CB_FP_PACKED
-      if (FULL) {
-        // rows q and q + 1 as packed pairs: per row the same unfused float
-        // operations as below, two rows per multiply and subtract
-        // instruction; the products only feed scalar adds
-        float2 acc2[RPL / 2], dz2[RPL / 2], iz2[RPL / 2];
+#define CB_FP_CELLS(S)                                                                     \
+  cb_fp_cells<RPL, S>(g, alphas, cells, mfast, vol, svz, dz2, iz2, acc2)
+      if (vb + 32 * RPL <= mid)
+        CB_FP_CELLS(BELOW);
+      else if (vb >= mid)
+        CB_FP_CELLS(ABOVE);
+      else // vb + 16 * RPL == mid
+        CB_FP_CELLS(HALVES);
+#undef CB_FP_CELLS
 #pragma unroll
-        for (int q = 0; q < RPL; q += 2) {
-          acc2[q / 2] = make_float2(0.0f, 0.0f);
-          dz2[q / 2] = make_float2(dzv[q], dzv[q + 1]);
-          iz2[q / 2] = make_float2(izv[q], izv[q + 1]);
-        }
-        for (int m = 1; m < mfast; m++) {
-          const float a0 = alphas[m - 1], a1 = alphas[m];
-          const int cell = cells[m - 1];
-          if (cell < 0)
-            continue;
-          const float *col = vol + i64(cell) * g.nz;
-          const float av = __fmul_rn(a0, inv_dz);
-          const float2 av2 = make_float2(av, av), a02 = make_float2(a0, a0),
-                       a12 = make_float2(a1, a1);
-#pragma unroll
-          for (int q = 0; q < RPL; q += 2) {
-            const float2 kz = mul2_rn(av2, dz2[q / 2]);
-            const int k0 = int(__fadd_rn(pzbz, kz.x)), k1 = int(__fadd_rn(pzbz, kz.y));
-            const float2 pl = mul2_rn(make_float2(vzq[q][k0], vzq[q + 1][k1]), iz2[q / 2]);
-            const float2 mz = make_float2(fmin_ref(pl.x, a1), fmin_ref(pl.y, a1));
-            const float2 lo = sub2_rn(mz, a02), hi = sub2_rn(a12, mz);
-            const float2 pk = mul2_rn(make_float2(__ldg(col + k0), __ldg(col + k1)), lo);
-            const float2 pn =
-                mul2_rn(make_float2(__ldg(col + k0 + dk[q]), __ldg(col + k1 + dk[q + 1])), hi);
-            acc2[q / 2] = add2_rn(acc2[q / 2],
-                                  make_float2(__fadd_rn(pk.x, pn.x), __fadd_rn(pk.y, pn.y)));
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < RPL; q += 2) {
-          acc[q] = acc2[q / 2].x;
-          acc[q + 1] = acc2[q / 2].y;
-        }
-      } else
-#endif
-      for (int m = 1; m < mfast; m++) {
-        const float a0 = alphas[m - 1], a1 = alphas[m];
-        const int cell = cells[m - 1];
-        if (cell < 0)
-          continue;
-        const float *col = vol + i64(cell) * g.nz;
-        const float av = __fmul_rn(a0, inv_dz);
-#pragma unroll
-        for (int q = 0; q < RPL; q++) {
-          if (!FULL && !vok[q])
-            continue;
-          const int k = int(__fadd_rn(pzbz, __fmul_rn(av, dzv[q])));
-          const float *ck = col + k;
-          const float mz = fmin_ref(__fmul_rn(vzq[q][k], izv[q]), a1);
-          acc[q] = __fadd_rn(acc[q], __fadd_rn(__fmul_rn(__ldg(ck), __fsub_rn(mz, a0)),
-                                               __fmul_rn(__ldg(ck + dk[q]), __fsub_rn(a1, mz))));
-        }
-      }
+      for (int q = 0; q < RPL; q++)
+        acc[q] = (q & 1) ? acc2[q / 2].y : acc2[q / 2].x;
       for (int m = max(mfast, 1); m < n; m++) {
         const float a0 = alphas[m - 1], a1 = alphas[m];
         const int cell = cells[m - 1];
@@ -413,7 +434,7 @@ __global__ void __launch_bounds__(kFpWarps * 32)
 #pragma unroll
       for (int q = 0; q < RPL; q++) {
         const int v = vb + q * 32 + lane;
-        if (v < g.nv) {
+        if (v >= 0 && v < g.nv) {
           const float dcv = g.dconv[i64(h) * g.nv + v];
           const float out = cb_fp_epi<EPI>(__fmul_rn(acc[q], dcv), rbase + v, e, ssq);
           // the SIRT / MLEM residual is the back projector's input: with
@@ -744,51 +765,60 @@ int cb_column_bands(const Geom &g, int2 *band, cudaStream_t st) {
 }
 
 namespace {
-// Rows per lane for nv rows: fewest idle lanes, then fewest passes.
-int cb_fp_rpl(int nv) {
-#ifdef CB_FP_FORCE_RPL
-  return CB_FP_FORCE_RPL;
-#endif
-  int best = 4;
-  long long best_waste = -1;
-  for (int r : {4, 8, 12}) {
-    const long long per = 32ll * r;
-    const long long waste = ((nv + per - 1) / per) * per - nv;
-    if (best_waste < 0 || waste < best_waste || (waste == best_waste && r > best)) {
-      best = r;
-      best_waste = waste;
-    }
+// Passes over the rows with r rows per lane: aligned to the first row above
+// the source (see cb_fp_kernel).
+struct FpRows {
+  int rpl, v0, np;
+};
+FpRows cb_fp_rows(const Geom &g, int r) {
+  FpRows p;
+  p.rpl = r;
+  p.v0 = g.mid - ((g.mid + 16 * r - 1) / (16 * r)) * 16 * r;
+  p.np = (g.nv - p.v0 + 32 * r - 1) / (32 * r);
+  return p;
+}
+// Rows per lane: the fewest instructions per cell, where a pass costs about
+// one more row per lane for reading the cell.
+FpRows cb_fp_rows(const Geom &g) {
+  if (g.tune_rpl >= 2 && g.tune_rpl <= 12 && g.tune_rpl % 2 == 0)
+    return cb_fp_rows(g, g.tune_rpl);
+  FpRows best = cb_fp_rows(g, 2);
+  for (int r = 4; r <= 12; r += 2) {
+    const FpRows p = cb_fp_rows(g, r);
+    if (p.np * (p.rpl + 1) <= best.np * (best.rpl + 1))
+      best = p;
   }
   return best;
 }
+
+} // namespace
+int cb_fp_rows_per_lane(const Geom &g) { return cb_fp_rows(g).rpl; }
+namespace {
 
 template <int EPI>
 void launch_cb_fp(const Geom &g, const float *vol, float *pix, const Epi &e, const int2 *hrange,
                   int grid, cudaStream_t st, int nb) {
   const size_t smem = cb_fp_smem(g);
   const int cap = g.nx + g.ny + 2;
-  const int r = (g.tune_rpl == 4 || g.tune_rpl == 8 || g.tune_rpl == 12) ? g.tune_rpl
-                                                                          : cb_fp_rpl(g.nv);
-  const bool full = g.nv % (32 * r) == 0;
-#define CB_FP_GO(R, F, B)                                                                  \
-  cb_fp_kernel<EPI, R, F, B><<<grid, kFpWarps * 32, smem, st>>>(g, vol, pix, e, hrange, cap, nb)
+  const FpRows p = cb_fp_rows(g);
+#define CB_FP_GO(R, B)                                                                     \
+  cb_fp_kernel<EPI, R, B><<<grid, kFpWarps * 32, smem, st>>>(g, vol, pix, e, hrange, cap, nb,  \
+                                                             p.v0, p.np)
+#define CB_FP_RPL(B)                                                                       \
+  (p.rpl == 2   ? CB_FP_GO(2, B)                                                            \
+   : p.rpl == 4 ? CB_FP_GO(4, B)                                                            \
+   : p.rpl == 6 ? CB_FP_GO(6, B)                                                            \
+   : p.rpl == 8 ? CB_FP_GO(8, B)                                                            \
+   : p.rpl == 10 ? CB_FP_GO(10, B)                                                          \
+                 : CB_FP_GO(12, B))
   if constexpr (EPI == EPI_STORE) {
     if (nb > 1) {
-      if (r == 12)
-        full ? CB_FP_GO(12, true, true) : CB_FP_GO(12, false, true);
-      else if (r == 8)
-        full ? CB_FP_GO(8, true, true) : CB_FP_GO(8, false, true);
-      else
-        full ? CB_FP_GO(4, true, true) : CB_FP_GO(4, false, true);
+      CB_FP_RPL(true);
       return;
     }
   }
-  if (r == 12)
-    full ? CB_FP_GO(12, true, false) : CB_FP_GO(12, false, false);
-  else if (r == 8)
-    full ? CB_FP_GO(8, true, false) : CB_FP_GO(8, false, false);
-  else
-    full ? CB_FP_GO(4, true, false) : CB_FP_GO(4, false, false);
+  CB_FP_RPL(false);
+#undef CB_FP_RPL
 #undef CB_FP_GO
 }
 } // namespace
@@ -796,14 +826,11 @@ void launch_cb_fp(const Geom &g, const float *vol, float *pix, const Epi &e, con
 int cb_prepare() {
   // the limit is the function's, not the plan's: the largest any plan uses
   const int fp = 200 * 1024;
-#define CB_FP_ALL(R, F)                                                                    \
-  (const void *)cb_fp_kernel<EPI_STORE, R, F, false>,                                       \
-      (const void *)cb_fp_kernel<EPI_NORM, R, F, false>,                                    \
-      (const void *)cb_fp_kernel<EPI_SIRT, R, F, false>,                                    \
-      (const void *)cb_fp_kernel<EPI_MLEM, R, F, false>,                                    \
-      (const void *)cb_fp_kernel<EPI_STORE, R, F, true>
-  const void *fps[] = {CB_FP_ALL(4, false), CB_FP_ALL(8, false), CB_FP_ALL(12, false),
-                       CB_FP_ALL(4, true),  CB_FP_ALL(8, true),  CB_FP_ALL(12, true),
+#define CB_FP_ALL(R)                                                                       \
+  (const void *)cb_fp_kernel<EPI_STORE, R, false>, (const void *)cb_fp_kernel<EPI_NORM, R, false>, \
+      (const void *)cb_fp_kernel<EPI_SIRT, R, false>,                                       \
+      (const void *)cb_fp_kernel<EPI_MLEM, R, false>, (const void *)cb_fp_kernel<EPI_STORE, R, true>
+  const void *fps[] = {CB_FP_ALL(2), CB_FP_ALL(4), CB_FP_ALL(6), CB_FP_ALL(8), CB_FP_ALL(10), CB_FP_ALL(12),
                        (const void *)cb_bp_scatter<1, false>,
                        (const void *)cb_bp_scatter<1, true>,
                        (const void *)cb_bp_scatter<2, false>,

@@ -55,12 +55,13 @@ struct Geom {
   const double2 *inv;     // na * nh: 1 / the ray's x and y spans (x = 0: the back
                           // projector takes no such ray, c2D.cpp:909-912)
   float neg0;             // -0.0f (see mul2_nz)
+  unsigned four;          // 4: bytes per float, as data (see cb_fp_cells)
   // nx * ny: per voxel column the back projector's band rows [x, y) that
   // stay inside the column for every ray crossing it (c2D.cpp:657-676)
   const int2 *colband;
   // ---- launch shapes chosen by ccpi_plan_autotune (0: the built-in choice)
   int tune_vw;            // parallel back projector: slices per lane (4, 8, 16)
-  int tune_rpl;           // cone forward projector: rows per lane (4, 8, 12)
+  int tune_rpl;           // cone forward projector: rows per lane (2, 4, .. 12)
   int tune_scatter;       // cone back projector: 1 ray-driven scatter, 0 voxel gather
 };
 

@@ -271,6 +271,7 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
       if (std::abs((double(dz[i]) - g.dz0) * g.inv_pitch - i) > 0.25)
         g.even_rows = 0;
     g.neg0 = -0.0f;
+    g.four = 4;
     g.dconv = upload(p, dconv);
     g.dz = upload(p, dz);
     g.iz = upload(p, iz);
@@ -1090,7 +1091,7 @@ int plan_autotune(ccpi_plan *p, cudaStream_t st, int *chosen) {
     p->bp_parts = pb_bp_tiles(p->g);
   } else if (rc == 0) {
     float t_best = 1e30f;
-    for (int rpl : {4, 8, 12}) {
+    for (int rpl : {0, 4, 6, 8, 10, 12}) { // 0: the built-in choice
       p->g.tune_rpl = rpl;
       const float t = timed([&] {
         cb_forward(p->g, vol, pix, EPI_STORE, none, p->hrange, p->fp_grid, st);
@@ -1121,7 +1122,7 @@ int plan_autotune(ccpi_plan *p, cudaStream_t st, int *chosen) {
   if (rc == 0 && !check_err(p))
     rc = 16;
   if (chosen) {
-    chosen[0] = p->g.kind == CCPI_PARALLEL ? p->fp_grid : p->g.tune_rpl;
+    chosen[0] = p->g.kind == CCPI_PARALLEL ? p->fp_grid : cb_fp_rows_per_lane(p->g);
     chosen[1] = p->g.kind == CCPI_PARALLEL ? p->g.tune_vw : p->g.tune_scatter;
   }
   if (e0)

@@ -21,6 +21,8 @@ int cb_column_bands(const Geom &g, int2 *band, cudaStream_t st);
 // projector forms them (Geom::inv)
 int cb_ray_spans(const Geom &g, double2 *inv, cudaStream_t st);
 size_t cb_fp_smem(const Geom &g);
+// detector rows per lane of the forward projector's passes
+int cb_fp_rows_per_lane(const Geom &g);
 // nb / nbatch: that many volumes and sinograms one after another, one launch
 // (EPI_STORE); the walk, row regimes and band limits are shared
 int cb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi &e,
