@@ -105,6 +105,8 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
   Geom &g = p->g;
   std::memset(&g, 0, sizeof(g));
   g.kind = gi->kind;
+  g.neg0 = -0.0f;
+  g.four = 4;
   g.na = gi->n_angles;
   g.nh = gi->n_h;
   g.nv = gi->n_v;
@@ -205,7 +207,7 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     g.vhi = upload(p, vhi);
     ok = ok && g.yoff && g.ioff && g.blen && g.map && g.vlo && g.vhi;
     p->fp_grid = pb_fp_ctas(g);
-    ok = ok && pb_prepare() == 0;
+    ok = ok && pb_prepare(g) == 0;
     p->bp_parts = pb_bp_tiles(g);
   } else {
     if (nv < 2) {
@@ -270,8 +272,6 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     for (int i = 0; i < nv; i++)
       if (std::abs((double(dz[i]) - g.dz0) * g.inv_pitch - i) > 0.25)
         g.even_rows = 0;
-    g.neg0 = -0.0f;
-    g.four = 4;
     g.dconv = upload(p, dconv);
     g.dz = upload(p, dz);
     g.iz = upload(p, iz);

@@ -25,6 +25,8 @@
 // Both kernels take fused epilogues (EpiMode): the SIRT and MLEM updates and
 // the FP64 sum of squares CGLS needs are applied to each output element
 // before it is stored, so no extra pass over HBM is spent on them.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -88,168 +90,6 @@ __device__ void pb_hrange(const Geom &g, double vx, double wx, double vy, double
   }
 }
 
-// Walk one non-axis-parallel ray through one block from the block's own
-// entry point (p2D.cpp:284-458), calling emit(column, length) per cell.
-// column = gx * ny + gy, or -1 outside the volume (the reference forms the
-// same flattened offset (x * ny + y) * nz and reads it).  The next x and y boundary
-// alphas are kept between steps and only the one crossed is re-evaluated,
-// with the reference's formula (b + i d - p2) / cos.
-template <class F>
-__device__ __forceinline__ void pb_walk_block(const Geom &g, double p2x, double p2y,
-                                              double c, double s, int bx0, int by0,
-                                              int nxb, int nyb, double vx, double vy,
-                                              F &emit) {
-  const double eps = double(kEps);
-  const double dx = g.size[0], dy = g.size[1];
-  const double xn = vx + double(nxb) * dx, yn = vy + double(nyb) * dy;
-  const double ic = 1.0 / c, is = 1.0 / s;
-  const double ax0 = (vx - p2x) * ic, ay0 = (vy - p2y) * is;
-  const double axn = (xn - p2x) * ic, ayn = (yn - p2y) * is;
-  const double amin = dmax(dmax(dmin(ax0, axn), dmin(ay0, ayn)), double(-g.d_conv));
-  const double amax = dmin(dmin(dmax(ax0, axn), dmax(ay0, ayn)), 0.0);
-  if (!(amin < amax - eps))
-    return;
-  const int sx = c > 0.0 ? 1 : -1, sy = s > 0.0 ? 1 : -1;
-  int x = 0, y = 0;
-  const bool x_face_first = !(sx > 0 && sy < 0); // octant (+,-) tests y first
-  auto cx = [&]() { return int(floor((p2x + amin * c - vx) / dx)); };
-  auto cy = [&]() { return int(floor((p2y + amin * s - vy) / dy)); };
-  const double axe = sx > 0 ? ax0 : axn; // entry through the x face
-  const double aye = sy > 0 ? ay0 : ayn; // entry through the y face
-  if (x_face_first) {
-    if (amin == axe) {
-      x = sx > 0 ? 0 : nxb - 1;
-      if (sx < 0 && sy < 0 && amin == ayn)
-        y = nyb - 1;
-      else
-        y = cy();
-    } else if (amin == aye) {
-      x = cx();
-      y = sy > 0 ? 0 : nyb - 1;
-    }
-  } else {
-    if (amin == aye) {
-      x = cx();
-      y = nyb - 1;
-    } else if (amin == axe) {
-      x = 0;
-      y = cy();
-    }
-  }
-  auto ax_at = [&](int i) { return (vx + double(i) * dx - p2x) * ic; };
-  auto ay_at = [&](int j) { return (vy + double(j) * dy - p2y) * is; };
-  const int ox = sx > 0 ? 1 : 0, oy = sy > 0 ? 1 : 0;
-  double nxa = ax_at(x + ox), nya = ay_at(y + oy);
-  double nxm = nxa - eps, nym = nya - eps;
-  double ap = amin;
-  const int ncol = g.nx * g.ny;
-  const int cstep_x = sx * g.ny;
-  int col = (bx0 + x) * g.ny + (by0 + y);
-  while ((sx > 0 ? x < nxb : x >= 0) && (sy > 0 ? y < nyb : y >= 0)) {
-    const int here = (unsigned(col) < unsigned(ncol)) ? col : -1;
-    float len;
-    if (nxa < nym) {
-      len = float(nxa - ap);
-      ap = nxa;
-      x += sx;
-      col += cstep_x;
-      nxa = ax_at(x + ox);
-      nxm = nxa - eps;
-    } else if (nya < nxm) {
-      len = float(nya - ap);
-      ap = nya;
-      y += sy;
-      col += sy;
-      nya = ay_at(y + oy);
-      nym = nya - eps;
-    } else {
-      const double mx = dmax(nxa, nya);
-      len = float(mx - ap);
-      ap = mx;
-      x += sx;
-      y += sy;
-      col += cstep_x + sy;
-      nxa = ax_at(x + ox);
-      nya = ay_at(y + oy);
-      nxm = nxa - eps;
-      nym = nya - eps;
-    }
-    emit(here, len);
-  }
-}
-
-// All cells of ray (a, h) in the reference's accumulation order: blocks in
-// (x-block, y-block) order, each applying the detector-column range rule.
-// `room` is called before each block (it may flush staged cells).
-template <class F, class R>
-__device__ void pb_trace_ray(const Geom &g, int a, int h, F &emit, R &room) {
-  const double eps = double(kEps);
-  const double c = g.cosA[a], s = g.sinA[a], hv = g.hpix[h];
-  const double p2x = c * g.det_x - s * hv;
-  const double p2y = s * g.det_x + c * hv;
-  const int nbx = (g.nx + kBlock - 1) / kBlock, nby = (g.ny + kBlock - 1) / kBlock;
-  const double dx = g.size[0], dy = g.size[1];
-  const int ncol = g.nx * g.ny;
-  if (fabs(c) < eps && fabs(s) < eps)
-    return;
-  for (int bxi = 0; bxi < nbx; bxi++) {
-    const int bx0 = bxi * kBlock, nxb = min(kBlock, g.nx - bx0);
-    const double vx = g.origin[0] + double(bx0) * dx;
-    const double wx = g.origin[0] + double(bx0 + nxb) * dx;
-    int by_lo = 0, by_hi = nby - 1;
-    int ix = 0;
-    if (fabs(c) < eps) {
-      // parallel to y: the block column that holds the ray by the floor rule
-      ix = int(floor((p2x - vx) / dx));
-      if (ix < 0 || ix >= nxb)
-        continue;
-    } else if (!(fabs(s) < eps)) {
-      // prefilter: block rows the ray can cross inside this block column
-      const double t = s / c;
-      const double ya = p2y + (vx - p2x) * t, yb = p2y + (wx - p2x) * t;
-      const double margin = 1e-3 * dy;
-      const double ylo = fmin(ya, yb) - margin, yhi = fmax(ya, yb) + margin;
-      const double bsz = double(kBlock) * dy;
-      const double flo = floor((ylo - g.origin[1]) / bsz);
-      const double fhi = floor((yhi - g.origin[1]) / bsz);
-      if (fhi < 0.0 || flo > double(nby - 1))
-        continue;
-      by_lo = flo < 0.0 ? 0 : int(flo);
-      by_hi = fhi > double(nby - 1) ? nby - 1 : int(fhi);
-    }
-    for (int byi = by_lo; byi <= by_hi; byi++) {
-      const int by0 = byi * kBlock, nyb = min(kBlock, g.ny - by0);
-      const double vy = g.origin[1] + double(by0) * dy;
-      const double wy = g.origin[1] + double(by0 + nyb) * dy;
-      int hmin, hmax;
-      pb_hrange(g, vx, wx, vy, wy, c, s, hmin, hmax);
-      if (h < hmin || h > hmax)
-        continue;
-      room();
-      if (fabs(c) < eps) {
-        const float len = float(dy);
-        for (int t = 0; t < nyb; t++) {
-          const int j = s < 0.0 ? nyb - 1 - t : t;
-          const int col = (bx0 + ix) * g.ny + by0 + j;
-          emit(unsigned(col) < unsigned(ncol) ? col : -1, len);
-        }
-      } else if (fabs(s) < eps) {
-        const int jy = int(floor((p2y - vy) / dy));
-        if (jy < 0 || jy >= nyb)
-          continue;
-        const float len = float(dx);
-        for (int t = 0; t < nxb; t++) {
-          const int i = c < 0.0 ? nxb - 1 - t : t;
-          const int col = (bx0 + i) * g.ny + by0 + jy;
-          emit(unsigned(col) < unsigned(ncol) ? col : -1, len);
-        }
-      } else {
-        pb_walk_block(g, p2x, p2y, c, s, bx0, by0, nxb, nyb, vx, vy, emit);
-      }
-    }
-  }
-}
-
 template <int EPI>
 __device__ __forceinline__ float fp_epilogue(float acc, i64 idx, const Epi &e, double &ssq) {
   if (EPI == EPI_NORM) {
@@ -276,18 +116,6 @@ __device__ void store_partial(double ssq, const Epi &e, bool add = false) {
   if (threadIdx.x == 0)
     e.partials[blockIdx.x] = add ? e.partials[blockIdx.x] + t : t;
 }
-
-// Staged cell lists: the warp-uniform walk emits (column, length) pairs into
-// the warp's slice of shared memory; the lanes then accumulate them in
-// order, four cells at a time with all loads issued before the adds.
-constexpr int kFpWarps = 8;  // warps of a CTA trace one detector column at 8 angles
-constexpr int kListCap = 256; // staged cells per warp
-constexpr int kBlockCells = 72; // most cells one ray has in one 32x32 block
-
-struct Cell {
-  int col;
-  float len;
-};
 
 // ---- forward, lane-parallel walk (row v -> slice v, nv and nz multiples of 4)
 //
@@ -324,7 +152,7 @@ struct LaneSmem {
 // nullptr) or written in y-block order for one block column.
 __device__ __forceinline__ int pb_column_blocks(const Geom &g, int h, double c, double s,
                                                 double p2x, double p2y, bool par_y, bool par_x,
-                                                int bxi, int *emit, int pos) {
+                                                int bxi, int *emit, int pos, int room) {
   const double dx = g.size[0], dy = g.size[1];
   const int nby = (g.ny + kBlock - 1) / kBlock;
   const int bx0 = bxi * kBlock, nxb = min(kBlock, g.nx - bx0);
@@ -362,11 +190,124 @@ __device__ __forceinline__ int pb_column_blocks(const Geom &g, int h, double c, 
       if (jy < 0 || jy >= nyb)
         continue;
     }
-    if (emit && pos + cnt < kMaxBlocks)
+    if (emit && pos + cnt < room)
       emit[pos + cnt] = (bxi << 16) | byi;
     cnt++;
   }
   return cnt;
+}
+
+// acc += x * l, unfused (see mul2_nz); add_cell_len: the same for x = 1.
+__device__ __forceinline__ void add_cell(float4 &acc, const float4 x, float l, float2 nz) {
+  const float2 w = make_float2(l, l);
+  const float2 a = add2_rn(make_float2(acc.x, acc.y), mul2_nz(make_float2(x.x, x.y), w, nz));
+  const float2 b = add2_rn(make_float2(acc.z, acc.w), mul2_nz(make_float2(x.z, x.w), w, nz));
+  acc = make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void add_cell(float &acc, float x, float l, float2) {
+  acc = __fadd_rn(acc, __fmul_rn(x, l));
+}
+__device__ __forceinline__ void add_cell_len(float4 &acc, float l) { add_len4(acc, l); }
+__device__ __forceinline__ void add_cell_len(float &acc, float l) { acc = __fadd_rn(acc, l); }
+
+// A ray as the block walks take it: direction, detector point, and what
+// follows from the direction.
+struct RayWalk {
+  double c, s, p2x, p2y, ic, is;
+  int sx, sy;
+  bool par_y, par_x, x_face_first; // octant (+,-) tests the y face first
+  __device__ RayWalk(double c_, double s_, double p2x_, double p2y_, bool py, bool px)
+      : c(c_), s(s_), p2x(p2x_), p2y(p2y_), ic(py ? 0.0 : 1.0 / c_), is(px ? 0.0 : 1.0 / s_),
+        sx(c_ > 0.0 ? 1 : -1), sy(s_ > 0.0 ? 1 : -1), par_y(py), par_x(px),
+        x_face_first(!(sx > 0 && sy < 0)) {}
+};
+
+// Walk ray W through block id = (x block << 16 | y block) from the block's own
+// entry point (p2D.cpp:284-458), calling put(column, length) per cell, which
+// counts the cells it keeps in n.  column = gx * ny + gy, formed beyond the
+// volume's edge as the reference forms it.  Returns false if n reached the
+// slot's size before the ray left the block.
+template <class F>
+__device__ __forceinline__ bool pb_walk_slot(const Geom &g, const RayWalk &W, int id, int &n,
+                                             F &&put) {
+  const double eps = double(kEps);
+  const double dx = g.size[0], dy = g.size[1];
+  const double c = W.c, s = W.s, p2x = W.p2x, p2y = W.p2y, ic = W.ic, is = W.is;
+  const int sx = W.sx, sy = W.sy, ox = sx > 0 ? 1 : 0, oy = sy > 0 ? 1 : 0;
+  const int bxi = id >> 16, byi = id & 0xffff;
+  const int bx0 = bxi * kBlock, nxb = min(kBlock, g.nx - bx0);
+  const int by0 = byi * kBlock, nyb = min(kBlock, g.ny - by0);
+  const double vx = g.origin[0] + double(bx0) * dx;
+  const double vy = g.origin[1] + double(by0) * dy;
+  if (W.par_y) {
+    const int ix = int(floor((p2x - vx) / dx));
+    const float len = float(dy);
+    for (int tt = 0; tt < nyb; tt++) {
+      const int jj = s < 0.0 ? nyb - 1 - tt : tt;
+      put((bx0 + ix) * g.ny + by0 + jj, len);
+    }
+    return true;
+  }
+  if (W.par_x) {
+    const int jy = int(floor((p2y - vy) / dy));
+    const float len = float(dx);
+    for (int tt = 0; tt < nxb; tt++) {
+      const int ii = c < 0.0 ? nxb - 1 - tt : tt;
+      put((bx0 + ii) * g.ny + by0 + jy, len);
+    }
+    return true;
+  }
+  const double xn = vx + double(nxb) * dx, yn = vy + double(nyb) * dy;
+  const double ax0 = (vx - p2x) * ic, ay0 = (vy - p2y) * is;
+  const double axn = (xn - p2x) * ic, ayn = (yn - p2y) * is;
+  const double amin = dmax(dmax(dmin(ax0, axn), dmin(ay0, ayn)), double(-g.d_conv));
+  const double amax = dmin(dmin(dmax(ax0, axn), dmax(ay0, ayn)), 0.0);
+  if (!(amin < amax - eps))
+    return true;
+  int x = 0, y = 0;
+  const double axe = sx > 0 ? ax0 : axn, aye = sy > 0 ? ay0 : ayn;
+  if (W.x_face_first) {
+    if (amin == axe) {
+      x = sx > 0 ? 0 : nxb - 1;
+      y = (sx < 0 && sy < 0 && amin == ayn) ? nyb - 1
+                                            : int(floor((p2y + amin * s - vy) / dy));
+    } else if (amin == aye) {
+      x = int(floor((p2x + amin * c - vx) / dx));
+      y = sy > 0 ? 0 : nyb - 1;
+    }
+  } else {
+    if (amin == aye) {
+      x = int(floor((p2x + amin * c - vx) / dx));
+      y = nyb - 1;
+    } else if (amin == axe) {
+      x = 0;
+      y = int(floor((p2y + amin * s - vy) / dy));
+    }
+  }
+  double nxa = (vx + double(x + ox) * dx - p2x) * ic;
+  double nya = (vy + double(y + oy) * dy - p2y) * is;
+  double ap = amin;
+  int col = (bx0 + x) * g.ny + (by0 + y);
+  const int cstep_x = sx * g.ny;
+  while ((sx > 0 ? x < nxb : x >= 0) && (sy > 0 ? y < nyb : y >= 0) && n < kSlotCap) {
+    const bool tx = nxa < nya - eps;
+    const bool ty = !tx && (nya < nxa - eps);
+    const bool both = !tx && !ty;
+    const double nxt = tx ? nxa : (ty ? nya : dmax(nxa, nya));
+    put(col, float(nxt - ap));
+    ap = nxt;
+    if (tx || both) {
+      x += sx;
+      col += cstep_x;
+      nxa = (vx + double(x + ox) * dx - p2x) * ic;
+    }
+    if (ty || both) {
+      y += sy;
+      col += sy;
+      nya = (vy + double(y + oy) * dy - p2y) * is;
+    }
+  }
+  return n < kSlotCap || !((sx > 0 ? x < nxb : x >= 0) && (sy > 0 ? y < nyb : y >= 0));
 }
 
 #ifndef PB_FP_MINB
@@ -431,7 +372,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
       for (int bbase = 0; bbase < nbx; bbase += 32) {
         const int bxi = bbase + lane;
         const int cnt =
-            bxi < nbx ? pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, nullptr, 0) : 0;
+            bxi < nbx ? pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, nullptr, 0, 0)
+                    : 0;
         int incl = cnt;
         for (int o = 1; o < 32; o <<= 1) {
           const int y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -439,7 +381,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
             incl += y;
         }
         if (cnt)
-          pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, S.blk, nblk + incl - cnt);
+          pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, S.blk, nblk + incl - cnt,
+                           kMaxBlocks);
         nblk += __shfl_sync(0xffffffffu, incl, 31);
       }
       if (nblk > kMaxBlocks) {
@@ -461,6 +404,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
           if (unsigned(col) < unsigned(ncol))
             myc[n++] = make_uint2(unsigned(col) * nz4, __float_as_uint(len));
         };
+        // pb_walk_slot, written out: as a call it costs this kernel 1 % in spills
         if (lane < kWalkLanes && j < nblk) {
           const int id = S.blk[j];
           const int bxi = id >> 16, byi = id & 0xffff;
@@ -617,71 +561,173 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
     store_partial<kLaneWarps>(ssq, e, v0 > 0);
 }
 
-// ---- forward, any row->slice mapping (p2D.cpp:63-213 cases 2, 4, default)
-template <int NS, int EPI>
-__global__ void __launch_bounds__(kFpWarps * 32) pb_fp_scalar(Geom g, const float *__restrict__ vol,
-                                                              float *__restrict__ pix, Epi e, int v0) {
-  __shared__ Cell lists[kFpWarps][kListCap];
+// ---- forward, few slices, or slices and rows that are not float4 rows
+//
+// A row's sum depends on its slice alone (p2D.cpp:63-213: every map type adds
+// col[map[v]] * length over the same cells), so lanes own slices, and a sum
+// is stored to every row of its slice.  G lanes share a ray, each with NQ x
+// VEC slices (float4 loads when a column is whole float4s); the 32 / G rays
+// of a warp are neighbouring angles of one detector column.  Every lane
+// walks one block of its group's ray at a time into its own slot; then each
+// group replays its slots in block order at its own pace.  The additions per
+// row are those of pb_fp_lanes, in the same order.
+//
+// Why: with one ray per warp, 16 rows of 192 x 192 x 16 kept 4 of 32 lanes
+// busy, and the form for other maps walked each ray with all lanes alike.
+template <int VEC> struct SliceVec;
+template <> struct SliceVec<4> {
+  typedef float4 T;
+};
+template <> struct SliceVec<1> {
+  typedef float T;
+};
+__device__ __forceinline__ float part(const float4 &a, int i) {
+  return i == 0 ? a.x : i == 1 ? a.y : i == 2 ? a.z : a.w;
+}
+__device__ __forceinline__ float part(const float &a, int) { return a; }
+
+// Words of one warp's staging: 32 slots, their counts, and the block lists of
+// its rays (room entries each).
+__host__ __device__ inline int group_words(int rays, int room) {
+  return (32 * kSlotCap * 2 + 32 + rays * room + 3) & ~3;
+}
+
+template <int VEC, int G, int NQ, int EPI>
+__global__ void __launch_bounds__(kLaneWarps * 32)
+    pb_fp_groups(Geom g, const float *__restrict__ vol, float *__restrict__ pix, Epi e, int z0,
+                 int room, int *err) {
+  typedef typename SliceVec<VEC>::T V;
+  constexpr int R = 32 / G; // rays of a warp
+  extern __shared__ unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  Cell *L = lists[wib];
+  const int l = lane & (G - 1), base = lane & ~(G - 1);
+  int *words = reinterpret_cast<int *>(smem_raw) + size_t(wib) * group_words(R, room);
+  uint2 *cells = reinterpret_cast<uint2 *>(words);
+  int *cnt = words + 32 * kSlotCap * 2;
+  int *blk = cnt + 32 + (lane / G) * room;
+  const double eps = double(kEps);
+  const int nbx = (g.nx + kBlock - 1) / kBlock;
+  const int ncol = g.nx * g.ny;
+  const float2 nz2 = make_float2(g.neg0, g.neg0);
+  // slices z0 + (q * G + l) * VEC + i
+  bool zok[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++)
+    zok[q] = z0 + (q * G + l) * VEC < g.nz;
+  const float *vz = vol + z0 + l * VEC;
   double ssq = 0.0;
-  int zmap[NS];
-#pragma unroll
-  for (int q = 0; q < NS; q++) {
-    const int v = v0 + q * 32 + lane;
-    zmap[q] = (v < g.nv) ? g.map[v] : -1;
-    if (zmap[q] >= g.nz)
-      zmap[q] = -1; // the reference reads past the column here
-  }
-  const int nat = (g.na + kFpWarps - 1) / kFpWarps;
-  const int ntiles = nat * g.nh;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int h = t / nat;
-    const int a = (t - h * nat) * kFpWarps + wib;
-    if (a >= g.na)
-      continue;
-    const int ray = a * g.nh + h;
-    float acc[NS];
-#pragma unroll
-    for (int q = 0; q < NS; q++)
-      acc[q] = 0.f;
-    int n = 0;
-    auto flush = [&]() {
+  const int nat = (g.na + kLaneWarps * R - 1) / (kLaneWarps * R);
+  const i64 ntiles = i64(nat) * g.nh;
+  for (i64 t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int h = int(t / nat);
+    const int a = (int(t - i64(h) * nat) * kLaneWarps + wib) * R + lane / G;
+    const int at = min(a, g.na - 1);
+    const double c = g.cosA[at], s = g.sinA[at], hv = g.hpix[h];
+    const double p2x = c * g.det_x - s * hv;
+    const double p2y = s * g.det_x + c * hv;
+    const bool par_y = fabs(c) < eps, par_x = !par_y && fabs(s) < eps;
+    const bool some = a < g.na && !(par_y && fabs(s) < eps);
+    V acc[NQ] = {};
+    // ---- the ray's blocks: x-block major, y-block ascending
+    int nblk = 0;
+    for (int b0 = 0; b0 < nbx; b0 += G) {
+      const int bxi = b0 + l;
+      const int n = (some && bxi < nbx)
+                        ? pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, nullptr, 0, 0)
+                        : 0;
+      int incl = n;
+      for (int o = 1; o < G; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o, G);
+        if (l >= o)
+          incl += y;
+      }
+      if (n)
+        pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, blk, nblk + incl - n, room);
+      nblk += __shfl_sync(0xffffffffu, incl, G - 1, G);
+    }
+    if (nblk > room) {
+      if (l == 0)
+        atomicExch(err, 3);
+      nblk = room;
+    }
+    __syncwarp();
+    const RayWalk W(c, s, p2x, p2y, par_y, par_x);
+    const int most = __reduce_max_sync(0xffffffffu, nblk);
+    for (int r0 = 0; r0 < most; r0 += G) {
+      // ---- one block per lane
+      uint2 *mine = cells + lane * kSlotCap;
+      int n = 0;
+      if (r0 + l < nblk && !pb_walk_slot(g, W, blk[r0 + l], n, [&](int col, float len) {
+            if (unsigned(col) < unsigned(ncol))
+              mine[n++] = make_uint2(unsigned(col), __float_as_uint(len));
+          }))
+        atomicExch(err, 3); // slot full before the ray left the block
+      cnt[lane] = n;
       __syncwarp();
-      for (int m = 0; m < n; m++) {
-        const Cell c1 = L[m];
-        if (c1.col < 0)
-          continue;
-        const float *colp = vol + i64(c1.col) * g.nz;
+      // ---- replay: up to four cells of the group's current slot a turn
+      int slot = base - 1, left = 0;
+      const uint2 *cl = cells;
+      while (true) {
+        while (left == 0 && slot < base + G - 1) {
+          slot++;
+          left = cnt[slot];
+          cl = cells + slot * kSlotCap;
+        }
+        if (!__any_sync(0xffffffffu, left > 0))
+          break;
+        const uint4 p0 = *reinterpret_cast<const uint4 *>(cl);
+        const uint4 p1 = *reinterpret_cast<const uint4 *>(cl + 2);
+        const unsigned o[4] = {p0.x, p0.z, p1.x, p1.z};
+        const float len[4] = {__uint_as_float(p0.y), __uint_as_float(p0.w), __uint_as_float(p1.y),
+                              __uint_as_float(p1.w)};
+        if (EPI == EPI_ONES) {
 #pragma unroll
-        for (int q = 0; q < NS; q++)
-          if (zmap[q] >= 0)
-            acc[q] = __fadd_rn(acc[q], __fmul_rn(__ldg(colp + zmap[q]), c1.len));
+          for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int q = 0; q < NQ; q++)
+              if (u < left)
+                add_cell_len(acc[q], len[u]);
+        } else {
+          V x[4][NQ];
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int q = 0; q < NQ; q++)
+              if (u < left && zok[q])
+                x[u][q] = __ldg(reinterpret_cast<const V *>(vz + i64(o[u]) * g.nz + q * G * VEC));
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int q = 0; q < NQ; q++)
+              if (u < left && zok[q])
+                add_cell(acc[q], x[u][q], len[u], nz2);
+        }
+        // a group that is done stays where it is: its reads stay in the slots
+        cl += left > 0 ? 4 : 0;
+        left = max(left - 4, 0);
       }
       __syncwarp();
-      n = 0;
-    };
-    auto emit = [&](int col, float len) {
-      if (lane == 0)
-        L[n] = Cell{col, len};
-      n++;
-    };
-    auto room = [&]() {
-      if (n > kListCap - kBlockCells)
-        flush();
-    };
-    pb_trace_ray(g, a, h, emit, room);
-    flush();
-    const i64 rbase = i64(ray) * g.nv;
+    }
+    // ---- store every slice's sum to its rows; rows of no slice are zero
+    if (a < g.na) {
+      const i64 rbase = (i64(a) * g.nh + h) * g.nv;
 #pragma unroll
-    for (int q = 0; q < NS; q++) {
-      const int v = v0 + q * 32 + lane;
-      if (v < g.nv)
-        pix[rbase + v] = fp_epilogue<EPI>(acc[q], rbase + v, e, ssq);
+      for (int q = 0; q < NQ; q++)
+#pragma unroll
+        for (int i = 0; i < VEC; i++) {
+          const int z = z0 + (q * G + l) * VEC + i;
+          if (z < g.nz)
+            for (int v = g.vlo[z]; v < g.vhi[z]; v++)
+              pix[rbase + v] = fp_epilogue<EPI>(part(acc[q], i), rbase + v, e, ssq);
+        }
+      if (z0 == 0 && g.map_type == 0)
+        for (int v = l; v < g.nv; v += G)
+          if (g.map[v] < 0 || g.map[v] >= g.nz)
+            pix[rbase + v] = fp_epilogue<EPI>(0.0f, rbase + v, e, ssq);
     }
   }
   if (EPI == EPI_NORM)
-    store_partial<kFpWarps>(ssq, e, v0 > 0);
+    store_partial<kLaneWarps>(ssq, e, z0 > 0);
 }
 
 // ---- backward
@@ -975,19 +1021,40 @@ __global__ void __launch_bounds__(256) pb_bp_scalar(Geom g, const float *__restr
     store_partial<8>(ssq, e);
 }
 
-// The lane-parallel forward kernel applies: row v <-> slice v, float4 rows,
-// float4 offsets of the columns fit 32 bits, and a ray's block list (at most
-// about nbx + nby entries) fits its staging area.
-bool pb_fp_vec4(const Geom &g) {
-  const int nblocks = (g.nx + kBlock - 1) / kBlock + (g.ny + kBlock - 1) / kBlock;
-  return g.map_type == 1 && (g.nv % 4) == 0 && (g.nz % 4) == 0 &&
-         (long long)g.nx * g.ny * (g.nz / 4) < (1ll << 32) && nblocks + 16 <= kMaxBlocks;
+// The one-ray-per-warp kernel applies: row v <-> slice v, float4 rows that
+// fill more than half a warp, float4 offsets of the columns fit 32 bits, and
+// a ray's block list (at most about nbx + nby entries) fits its staging area.
+int pb_block_room(const Geom &g) {
+  return (g.nx + kBlock - 1) / kBlock + (g.ny + kBlock - 1) / kBlock + 16;
+}
+bool pb_fp_one_ray(const Geom &g) {
+  return g.map_type == 1 && (g.nv % 4) == 0 && (g.nz % 4) == 0 && g.nv > 64 &&
+         (long long)g.nx * g.ny * (g.nz / 4) < (1ll << 32) && pb_block_room(g) <= kMaxBlocks;
+}
+
+// Lanes per ray and slices per lane for the others: the fewest lanes that
+// hold the rows' slices (slices past the last row's need no sum), then up to
+// 2 float4 or 4 floats per lane and launch.
+struct GroupShape {
+  int vec, g, nq, slices;
+};
+GroupShape group_shape(const Geom &g) {
+  GroupShape s;
+  s.slices = g.map_type == 1 ? std::min(g.nv, g.nz) : g.nz;
+  s.vec = g.nz % 4 == 0 ? 4 : 1;
+  const int lanes = (s.slices + s.vec - 1) / s.vec;
+  s.g = lanes <= 4 && s.vec == 4 ? 4 : lanes <= 8 && s.vec == 4 ? 8 : lanes <= 16 ? 16 : 32;
+  s.nq = lanes <= 32 ? 1 : lanes <= 64 || s.vec == 4 ? 2 : 4;
+  return s;
+}
+size_t group_smem(const Geom &g, int lanes) {
+  return size_t(kLaneWarps) * group_words(32 / lanes, pb_block_room(g)) * 4;
 }
 
 template <int EPI>
 int launch_fp(const Geom &g, const float *vol, float *pix, const Epi &e, int grid, int *err,
               cudaStream_t st) {
-  if (pb_fp_vec4(g)) {
+  if (pb_fp_one_ray(g)) {
     const size_t smem = sizeof(LaneSmem) * kLaneWarps;
     for (int v0 = 0; v0 < g.nv; v0 += 256) {
       if (g.nv - v0 > 128)
@@ -995,16 +1062,36 @@ int launch_fp(const Geom &g, const float *vol, float *pix, const Epi &e, int gri
       else
         pb_fp_lanes<1, EPI><<<grid, kLaneWarps * 32, smem, st>>>(g, vol, pix, e, v0, err);
     }
-  } else if (EPI != EPI_ONES) {
-    for (int v0 = 0; v0 < g.nv; v0 += 256) {
-      const int left = g.nv - v0;
-      if (left > 128)
-        pb_fp_scalar<8, EPI><<<grid, kFpWarps * 32, 0, st>>>(g, vol, pix, e, v0);
-      else if (left > 32)
-        pb_fp_scalar<4, EPI><<<grid, kFpWarps * 32, 0, st>>>(g, vol, pix, e, v0);
+    return 0;
+  }
+  const GroupShape s = group_shape(g);
+  const size_t smem = group_smem(g, s.g);
+  const int room = pb_block_room(g);
+  for (int z0 = 0; z0 < s.slices; z0 += s.g * s.nq * s.vec) {
+#define PB_GROUPS(V, L, Q)                                                                 \
+  pb_fp_groups<V, L, Q, EPI><<<grid, kLaneWarps * 32, smem, st>>>(g, vol, pix, e, z0, room, err)
+    if (s.vec == 4) {
+      if (s.g == 4)
+        PB_GROUPS(4, 4, 1);
+      else if (s.g == 8)
+        PB_GROUPS(4, 8, 1);
+      else if (s.g == 16)
+        PB_GROUPS(4, 16, 1);
+      else if (s.nq == 1)
+        PB_GROUPS(4, 32, 1);
       else
-        pb_fp_scalar<1, EPI><<<grid, kFpWarps * 32, 0, st>>>(g, vol, pix, e, v0);
+        PB_GROUPS(4, 32, 2);
+    } else {
+      if (s.g == 16)
+        PB_GROUPS(1, 16, 1);
+      else if (s.nq == 1)
+        PB_GROUPS(1, 32, 1);
+      else if (s.nq == 2)
+        PB_GROUPS(1, 32, 2);
+      else
+        PB_GROUPS(1, 32, 4);
     }
+#undef PB_GROUPS
   }
   return 0;
 }
@@ -1099,8 +1186,6 @@ int pb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi 
                int grid, int *err, cudaStream_t st) {
   switch (mode) {
   case EPI_ONES:
-    if (!pb_fp_vec4(g))
-      return 3; // no ones form for this geometry: the caller projects a ones volume
     return launch_fp<EPI_ONES>(g, vol, pix, e, grid, err, st);
   case EPI_STORE:
     return launch_fp<EPI_STORE>(g, vol, pix, e, grid, err, st);
@@ -1116,22 +1201,42 @@ int pb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi 
 
 // Opt the forward kernels into their shared memory (done once, outside any
 // graph capture).
-int pb_prepare() {
-  const int smem = int(sizeof(LaneSmem) * kLaneWarps);
-  const void *fns[] = {(const void *)pb_fp_lanes<1, EPI_STORE>, (const void *)pb_fp_lanes<2, EPI_STORE>,
-                       (const void *)pb_fp_lanes<1, EPI_NORM>,  (const void *)pb_fp_lanes<2, EPI_NORM>,
-                       (const void *)pb_fp_lanes<1, EPI_SIRT>,  (const void *)pb_fp_lanes<2, EPI_SIRT>,
-                       (const void *)pb_fp_lanes<1, EPI_MLEM>,  (const void *)pb_fp_lanes<2, EPI_MLEM>,
-                       (const void *)pb_fp_lanes<1, EPI_ONES>,  (const void *)pb_fp_lanes<2, EPI_ONES>};
-  for (const void *f : fns)
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return 1;
-  return 0;
+int pb_prepare(const Geom &g) {
+  if (group_smem(g, group_shape(g).g) > 200 * 1024)
+    return 1;
+  bool ok = true;
+  auto allow = [&](const void *f, int smem) {
+    ok = ok &&
+         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+  };
+#define PB_ALL(E)                                                                          \
+  {                                                                                        \
+    for (const void *f : {(const void *)pb_fp_lanes<1, E>, (const void *)pb_fp_lanes<2, E>}) \
+      allow(f, int(sizeof(LaneSmem) * kLaneWarps));                                         \
+    for (const void *f :                                                                    \
+         {(const void *)pb_fp_groups<4, 4, 1, E>, (const void *)pb_fp_groups<4, 8, 1, E>,    \
+          (const void *)pb_fp_groups<4, 16, 1, E>, (const void *)pb_fp_groups<4, 32, 1, E>,  \
+          (const void *)pb_fp_groups<4, 32, 2, E>, (const void *)pb_fp_groups<1, 16, 1, E>,  \
+          (const void *)pb_fp_groups<1, 32, 1, E>, (const void *)pb_fp_groups<1, 32, 2, E>,  \
+          (const void *)pb_fp_groups<1, 32, 4, E>})                                          \
+      allow(f, 200 * 1024);                                                                 \
+  }
+  PB_ALL(EPI_STORE)
+  PB_ALL(EPI_NORM)
+  PB_ALL(EPI_SIRT)
+  PB_ALL(EPI_MLEM)
+  PB_ALL(EPI_ONES)
+#undef PB_ALL
+  return ok ? 0 : 1;
 }
 
+// As many CTAs as are resident (five, or three by the groups' staging), each
+// walking the tiles in order.
 int pb_fp_ctas(const Geom &g) {
-  const long long tiles = (long long)((g.na + kLaneWarps - 1) / kLaneWarps) * g.nh;
-  return int(tiles < 148 * PB_FP_CTAS_PER_SM ? tiles : 148 * PB_FP_CTAS_PER_SM);
+  const bool one = pb_fp_one_ray(g);
+  const int rays = one ? kLaneWarps : kLaneWarps * (32 / group_shape(g).g);
+  const long long tiles = (long long)((g.na + rays - 1) / rays) * g.nh;
+  return int(std::min<long long>(tiles, 148 * (one ? PB_FP_CTAS_PER_SM : 3)));
 }
 
 int pb_backward(const Geom &g, const float *pix, float *vol, int mode, const Epi &e,
