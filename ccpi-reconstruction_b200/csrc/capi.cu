@@ -322,7 +322,10 @@ struct DevBuf {
     return ccpi::cuda_ok(cudaMalloc(&p, bytes ? bytes : 4), "device allocation");
   }
   float *f() { return static_cast<float *>(p); }
+  float *at(size_t bytes) { return reinterpret_cast<float *>(static_cast<char *>(p) + bytes); }
 };
+
+size_t up256(size_t n) { return (n + 255) & ~size_t(255); }
 
 struct PlanHolder {
   ccpi_plan *p = nullptr;
@@ -340,27 +343,32 @@ int solve_on_host_data(HostGeometry &G, int alg, const float *sino_host, bool ra
     return 2;
   const i64 V = P.p->nvox, Pn = P.p->npix;
   const i64 raw = raw_parallel ? i64(na) * nv * nh : Pn;
-  DevBuf draw, dsino, dx;
-  if ((raw_parallel && !draw.alloc(raw * 4)) || !dsino.alloc(Pn * 4) || !dx.alloc(V * 4))
+  // the call's buffers and the solver's workspace, one allocation
+  const size_t ws_bytes = ccpi::solve_workspace_bytes(P.p, alg, niter);
+  const size_t at_x = up256(Pn * 4), at_ws = at_x + up256(V * 4), at_raw = at_ws + up256(ws_bytes);
+  DevBuf all;
+  if (!all.alloc(at_raw + (raw_parallel ? raw * 4 : 0)))
     return 2;
+  float *dsino = all.at(0), *dx = all.at(at_x), *draw = all.at(at_raw);
   cudaStream_t st = 0;
-  if (!ccpi::cuda_ok(cudaMemcpyAsync(raw_parallel ? draw.p : dsino.p, sino_host, raw * 4,
+  if (!ccpi::cuda_ok(cudaMemcpyAsync(raw_parallel ? draw : dsino, sino_host, raw * 4,
                                      cudaMemcpyHostToDevice, st),
                      "upload sinogram"))
     return 2;
   if (raw_parallel)
-    ccpi::k_pack_parallel(draw.f(), dsino.f(), na, nv, nh, G.nv_pad, G.v_offset, st);
+    ccpi::k_pack_parallel(draw, dsino, na, nv, nh, G.nv_pad, G.v_offset, st);
   if (x0) {
-    if (!ccpi::cuda_ok(cudaMemcpyAsync(dx.p, x0, V * 4, cudaMemcpyHostToDevice, st),
+    if (!ccpi::cuda_ok(cudaMemcpyAsync(dx, x0, V * 4, cudaMemcpyHostToDevice, st),
                        "upload x0"))
       return 2;
   } else {
-    cudaMemsetAsync(dx.p, 0, V * 4, st);
+    cudaMemsetAsync(dx, 0, V * 4, st);
   }
-  const int rc = ccpi::solve(P.p, alg, dsino.f(), dx.f(), niter, lambda, norms, 0, nullptr, 0, st);
+  const int rc = ccpi::solve(P.p, alg, dsino, dx, niter, lambda, norms, 0, all.at(at_ws),
+                             ws_bytes, st);
   if (rc)
     return rc;
-  if (!ccpi::cuda_ok(cudaMemcpy(volume, dx.p, V * 4, cudaMemcpyDeviceToHost), "download volume"))
+  if (!ccpi::cuda_ok(cudaMemcpy(volume, dx, V * 4, cudaMemcpyDeviceToHost), "download volume"))
     return 2;
   return 0;
 }
@@ -820,19 +828,24 @@ int ccpi_reconstruct_flags(const ccpi_geometry *geometry, int alg, const float *
       ccpi::set_cone_backprojector(P.p, 1))
     return 1;
   const i64 V = P.p->nvox, Pn = P.p->npix;
-  DevBuf dsino, dx;
-  if (!dsino.alloc(Pn * 4) || !dx.alloc(V * 4))
+  // the call's buffers and the solver's workspace, one allocation
+  const size_t ws_bytes = ccpi::solve_workspace_bytes(P.p, alg, niter);
+  const size_t at_x = up256(Pn * 4), at_ws = at_x + up256(V * 4);
+  DevBuf all;
+  if (!all.alloc(at_ws + ws_bytes))
     return 2;
+  float *dsino = all.at(0), *dx = all.at(at_x);
   cudaStream_t st = 0;
-  if (!ccpi::cuda_ok(cudaMemcpyAsync(dsino.p, sino, Pn * 4, cudaMemcpyHostToDevice, st),
+  if (!ccpi::cuda_ok(cudaMemcpyAsync(dsino, sino, Pn * 4, cudaMemcpyHostToDevice, st),
                      "ccpi_reconstruct: upload sinogram"))
     return 2;
-  cudaMemsetAsync(dx.p, 0, V * 4, st);
+  cudaMemsetAsync(dx, 0, V * 4, st);
   const int rc =
-      ccpi::solve(P.p, alg, dsino.f(), dx.f(), niter, regularize, norms, 0, nullptr, 0, st);
+      ccpi::solve(P.p, alg, dsino, dx, niter, regularize, norms, 0, all.at(at_ws),
+                  ws_bytes, st);
   if (rc)
     return rc;
-  if (!ccpi::cuda_ok(cudaMemcpy(volume, dx.p, V * 4, cudaMemcpyDeviceToHost),
+  if (!ccpi::cuda_ok(cudaMemcpy(volume, dx, V * 4, cudaMemcpyDeviceToHost),
                      "ccpi_reconstruct: download volume"))
     return 2;
   return 0;
