@@ -493,6 +493,9 @@ template <int RPL, int SIDE>
 __device__ __forceinline__ void cb_scatter_cell(const Geom &g, float a0, float a1, float *vcol,
                                                 unsigned vz, int side, const float (&dzv)[RPL],
                                                 const float (&izv)[RPL], const float (&p)[RPL]) {
+  // the source then lies between two groups of rows or between lanes 15 and
+  // 16 of one (three rows per lane would put it after lane 23)
+  static_assert(RPL == 1 || RPL % 2 == 0, "rows per lane: 1 or pairs");
   constexpr unsigned kMagic = 0x4b000000u; // bits of 2^23
   const float2 nz = make_float2(g.neg0, g.neg0);
   const float2 pz = make_float2(g.pzbz, g.pzbz), big = make_float2(8388608.0f, 8388608.0f);
@@ -765,11 +768,10 @@ RowPasses row_passes(const Geom &g, int r) {
 }
 // Rows per lane of the scatter: as for the forward projector, with a pass's
 // reading of the cell and its band worth two rows per lane.  512^3 with 768
-// rows: 476 ms with 2 rows per lane, 401 with 3, 364 with 4, 326 with 6, 320
-// with 8.
+// rows: 476 ms with 2 rows per lane, 364 with 4, 326 with 6, 320 with 8.
 RowPasses cb_scatter_rows(const Geom &g) {
   RowPasses best = row_passes(g, 1);
-  for (int r : {2, 3, 4, 6, 8}) {
+  for (int r : {2, 4, 6, 8}) {
     const RowPasses p = row_passes(g, r);
     if (p.np * (p.rpl + 2) <= best.np * (best.rpl + 2))
       best = p;
@@ -796,9 +798,6 @@ int cb_backward_scatter(const Geom &g, const float *pix, float *vol, int pre,
     break;
   case 2:
     CB_SC_GO(2);
-    break;
-  case 3:
-    CB_SC_GO(3);
     break;
   case 4:
     CB_SC_GO(4);
@@ -878,8 +877,6 @@ int cb_prepare() {
                        (const void *)cb_bp_scatter<1, true>,
                        (const void *)cb_bp_scatter<2, false>,
                        (const void *)cb_bp_scatter<2, true>,
-                       (const void *)cb_bp_scatter<3, false>,
-                       (const void *)cb_bp_scatter<3, true>,
                        (const void *)cb_bp_scatter<4, false>,
                        (const void *)cb_bp_scatter<4, true>,
                        (const void *)cb_bp_scatter<6, false>,

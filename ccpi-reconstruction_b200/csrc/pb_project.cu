@@ -947,6 +947,9 @@ __global__ void __launch_bounds__(256, NP * VW <= 16 ? 4 : (NP * VW <= 32 ? 3 : 
 }
 
 // Scalar over z, any row->slice mapping (calc_ah_z cases, p2D.cpp:613-773).
+// Bound: instruction issue.  With the map type decided per ray and every row
+// address formed anew it took 115 issue slots per warp and ray (256 x 256 x 64
+// from 128 rows, 300 angles: 5.10 ms).
 template <int NP, int EPI>
 __global__ void __launch_bounds__(256) pb_bp_scalar(Geom g, const float *__restrict__ pix,
                                                     float *__restrict__ vol, Epi e, int tw,
@@ -955,6 +958,7 @@ __global__ void __launch_bounds__(256) pb_bp_scalar(Geom g, const float *__restr
   const int ntx = (g.nx + tw - 1) / tw;
   const int tx0 = (blockIdx.x % ntx) * tw, ty0 = (blockIdx.x / ntx) * th;
   const int npairs = tw * th * g.nz;
+  const bool wide = g.nv % max(g.map_type, 1) == 0; // a slice's rows are aligned
   float acc[NP];
   int pcol[NP], pz[NP];
 #pragma unroll
@@ -975,35 +979,39 @@ __global__ void __launch_bounds__(256) pb_bp_scalar(Geom g, const float *__restr
         continue;
       const int z = pz[k];
       const BpEntry *E = ent + pcol[k] * kBpAngles;
-      for (int ai = 0; ai < na_chunk; ai++) {
-        const int cnt = E[ai].cnt;
-        const float *row = pix + (i64(a0 + ai) * g.nh + E[ai].h0) * g.nv;
-        for (int r = 0; r < cnt; r++) {
-          const float w = E[ai].w[r];
-          const float *p = row + i64(r) * g.nv;
-          switch (g.map_type) {
-          case 1:
-            if (z < g.nv)
-              acc[k] = __fadd_rn(acc[k], __fmul_rn(p[z], w));
-            break;
-          case 2:
-            if (2 * z + 1 < g.nv)
-              acc[k] = __fadd_rn(acc[k], __fmul_rn(__fadd_rn(p[2 * z], p[2 * z + 1]), w));
-            break;
-          case 4:
-            if (4 * z + 3 < g.nv) {
-              const float t = __fadd_rn(__fadd_rn(__fadd_rn(p[4 * z], p[4 * z + 1]), p[4 * z + 2]),
-                                        p[4 * z + 3]);
-              acc[k] = __fadd_rn(acc[k], __fmul_rn(t, w));
-            }
-            break;
-          default:
-            for (int v = g.vlo[z]; v < g.vhi[z]; v++)
-              acc[k] = __fadd_rn(acc[k], __fmul_rn(p[v], w));
-            break;
-          }
+      float t = acc[k];
+      // every ray's row at offset off of its detector column; the map type
+      // is decided once per chunk of angles
+      auto sweep = [&](int off, auto &&add) {
+        for (int ai = 0; ai < na_chunk; ai++) {
+          const int cnt = E[ai].cnt;
+          const float *p = pix + (i64(a0 + ai) * g.nh + E[ai].h0) * g.nv + off;
+          for (int r = 0; r < cnt; r++, p += g.nv)
+            add(p, E[ai].w[r]);
         }
+      };
+      if (g.map_type == 1 && z < g.nv)
+        sweep(z, [&](const float *p, float w) { t = __fadd_rn(t, __fmul_rn(__ldg(p), w)); });
+      else if (g.map_type == 2 && 2 * z + 1 < g.nv)
+        sweep(2 * z, [&](const float *p, float w) {
+          const float2 x = wide ? __ldg(reinterpret_cast<const float2 *>(p))
+                                : make_float2(__ldg(p), __ldg(p + 1));
+          t = __fadd_rn(t, __fmul_rn(__fadd_rn(x.x, x.y), w));
+        });
+      else if (g.map_type == 4 && 4 * z + 3 < g.nv)
+        sweep(4 * z, [&](const float *p, float w) {
+          const float4 x = wide ? __ldg(reinterpret_cast<const float4 *>(p))
+                                : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+          t = __fadd_rn(t, __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn(x.x, x.y), x.z), x.w), w));
+        });
+      else if (g.map_type == 0) {
+        const int lo = g.vlo[z], n = g.vhi[z] - lo;
+        sweep(lo, [&](const float *p, float w) {
+          for (int v = 0; v < n; v++)
+            t = __fadd_rn(t, __fmul_rn(__ldg(p + v), w));
+        });
       }
+      acc[k] = t;
     }
   }
   double ssq = 0.0;

@@ -46,3 +46,25 @@ def test_tiles_equal_the_oracle(name, cuda):
         both = p.backward_batch(t, torch.empty((2,) + p.shape, device=cuda)).cpu().numpy()
         assert np.array_equal(both[0], ref, equal_nan=True)
         assert np.array_equal(both[1], O.backward(g, pix[1]), equal_nan=True)
+
+
+@pytest.mark.parametrize("nv", [6, 24, 32, 40, 64, 96, 100, 128, 160, 192, 200, 256, 288, 300])
+def test_scatter_at_every_row_count(nv, cuda):
+    """The scatter's passes of rows (1 to 8 per lane, split by the source or
+    not): within the projector tolerance of the oracle."""
+    import torch
+    from ccpi.reconstruction.device import Plan
+    g = O.cone_geometry((26, 21, 30), 1.0, 11, 37, 1.1, 60.0, 60.0, n_det_v=nv)
+    # rows over the same height, the source above or below the middle
+    g.v_pixels = (np.arange(nv) - (nv - 1) / 2.0) * (34.0 / nv) + (0.1 if nv % 3 else 3.2)
+    p = Plan("cone", g.angles, g.h_pixels, g.v_pixels, g.origin, g.size, g.shape,
+             source=g.source, detector_x=g.detector_x)
+    rng = np.random.default_rng(nv)
+    pix = rng.random(g.sino_shape).astype(np.float32)
+    ref = O.backward(g, pix)
+    p.set_cone_backprojector(1)
+    out = p.backward(torch.from_numpy(pix).to(cuda)).cpu().numpy()
+    assert np.abs(out - ref).max() <= 1e-5 * np.abs(ref).max()
+    vol = rng.random(g.shape).astype(np.float32)
+    assert np.array_equal(p.forward(torch.from_numpy(vol).to(cuda)).cpu().numpy(),
+                          O.forward(g, vol))
