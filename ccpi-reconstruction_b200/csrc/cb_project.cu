@@ -480,22 +480,20 @@ __global__ void __launch_bounds__(kFpWarps * 32)
 // target was measured slower on every geometry: 1250 against 1012 ms at
 // 512^3, 69 against 58 ms at 256^3.)
 
-// One cell whose rows of this pass all lie in the column's band, with every
-// slice k and its neighbour inside the column (cb_row_regimes).  Rows j and
-// j + 1 as packed pairs; a pair on one slice adds its two sums, in row order,
-// and a weight of zero (the row does not cross the plane) adds nothing.
 // An address computed in asm has lost its state space: name it here.
 __device__ __forceinline__ void red_add(const float *p, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
 
-template <int RPL, int SIDE>
+// One cell whose rows of this pass all lie in the column's band, with every
+// slice k and its neighbour inside the column (cb_row_regimes).  Rows j and
+// j + 1 as packed pairs; a pair on one slice adds its two sums, in row order,
+// and a weight of zero (the row does not cross the plane) adds nothing.  IDLE:
+// many rows lie outside the detector, and their sums add nothing either.
+template <int RPL, int SIDE, bool IDLE>
 __device__ __forceinline__ void cb_scatter_cell(const Geom &g, float a0, float a1, float *vcol,
                                                 unsigned vz, int side, const float (&dzv)[RPL],
                                                 const float (&izv)[RPL], const float (&p)[RPL]) {
-  // the source then lies between two groups of rows or between lanes 15 and
-  // 16 of one (three rows per lane would put it after lane 23)
-  static_assert(RPL == 1 || RPL % 2 == 0, "rows per lane: 1 or pairs");
   constexpr unsigned kMagic = 0x4b000000u; // bits of 2^23
   const float2 nz = make_float2(g.neg0, g.neg0);
   const float2 pz = make_float2(g.pzbz, g.pzbz), big = make_float2(8388608.0f, 8388608.0f);
@@ -507,7 +505,8 @@ __device__ __forceinline__ void cb_scatter_cell(const Geom &g, float a0, float a
   // D: the neighbour's step, 0 for the lane's own
   auto add = [&](unsigned k, int D, float s1, float s2) {
     const float *c = at_wide(k, g.four, col);
-    red_add(c, s1);
+    if (!IDLE || s1 != 0.0f)
+      red_add(c, s1);
     if (s2 != 0.0f)
       red_add(D == 0 ? at_wide(k, g.four, ncol) : c + D, s2);
   };
@@ -565,7 +564,9 @@ __global__ void __launch_bounds__(kFpWarps * 32, 8)
   const int nz = g.nz, nzm1 = g.nz - 1, mid = g.mid;
   const float pzbz = g.pzbz, pzbz1 = g.pzbz1, inv_dz = g.inv_dz;
   const unsigned vz = unsigned(__cvta_generic_to_shared(svz));
-  const int side = lane < 16 ? -1 : 1; // of a pass with the source in its middle
+  // The lane's side of the source in the 64 rows (one row per lane: 32) that
+  // hold row 16 * RPL, where a pass with the source in its middle has it.
+  const int side = lane < (RPL == 1 ? 16 : 16 * RPL % 64 / 2) ? -1 : 1;
   for (int ray = blockIdx.x * kFpWarps + wib; ray < nrays; ray += gridDim.x * kFpWarps) {
     const int a = ray / g.nh, h = ray - a * g.nh;
     const int2 hr = hrange[a];
@@ -601,6 +602,10 @@ __global__ void __launch_bounds__(kFpWarps * 32, 8)
         p[j] = (PRE || !vok[j]) ? y : __fmul_rn(y, g.dconv[i64(h) * g.nv + v]);
       }
       const int r0 = max(vb, 0), r1 = min(vb + 32 * RPL, g.nv); // the pass's rows
+      // with more than a sixteenth of its rows outside the detector a pass
+      // tests every sum for zero (288 rows in a pass of 320: 8.5 against
+      // 9.3 ms; 256^3 with every row inside: 22.5 against 20.6 ms)
+      const bool idle = r1 - r0 < 30 * RPL;
       // the crossed column's band, loaded one cell ahead
       int2 band_next = cells[0] >= 0 ? g.colband[cells[0]] : make_int2(0, 0);
       for (int m = 1; m < n; m++) {
@@ -613,7 +618,9 @@ __global__ void __launch_bounds__(kFpWarps * 32, 8)
         const float a0 = alphas[m - 1], a1 = alphas[m];
         float *col = vol + i64(cell) * nz;
         if (m < mfast && r0 >= band.x && r1 <= band.y) {
-#define CB_SC_CELL(S) cb_scatter_cell<RPL, S>(g, a0, a1, col, vz, side, dzv, izv, p)
+#define CB_SC_CELL(S)                                                                      \
+  (idle ? cb_scatter_cell<RPL, S, true>(g, a0, a1, col, vz, side, dzv, izv, p)                \
+        : cb_scatter_cell<RPL, S, false>(g, a0, a1, col, vz, side, dzv, izv, p))
           if (vb + 32 * RPL <= mid)
             CB_SC_CELL(BELOW);
           else if (vb >= mid)
@@ -768,10 +775,11 @@ RowPasses row_passes(const Geom &g, int r) {
 }
 // Rows per lane of the scatter: as for the forward projector, with a pass's
 // reading of the cell and its band worth two rows per lane.  512^3 with 768
-// rows: 476 ms with 2 rows per lane, 364 with 4, 326 with 6, 320 with 8.
+// rows: 476 ms with 2 rows per lane, 401 with 3, 364 with 4, 326 with 6,
+// 320 with 8; 288 rows 8.5 ms with 10, 9.6 with two passes of 6.
 RowPasses cb_scatter_rows(const Geom &g) {
   RowPasses best = row_passes(g, 1);
-  for (int r : {2, 4, 6, 8}) {
+  for (int r : {2, 3, 4, 6, 8, 10}) {
     const RowPasses p = row_passes(g, r);
     if (p.np * (p.rpl + 2) <= best.np * (best.rpl + 2))
       best = p;
@@ -799,14 +807,20 @@ int cb_backward_scatter(const Geom &g, const float *pix, float *vol, int pre,
   case 2:
     CB_SC_GO(2);
     break;
+  case 3:
+    CB_SC_GO(3);
+    break;
   case 4:
     CB_SC_GO(4);
     break;
   case 6:
     CB_SC_GO(6);
     break;
-  default:
+  case 8:
     CB_SC_GO(8);
+    break;
+  default:
+    CB_SC_GO(10);
   }
 #undef CB_SC_GO
   return 0;
@@ -877,12 +891,16 @@ int cb_prepare() {
                        (const void *)cb_bp_scatter<1, true>,
                        (const void *)cb_bp_scatter<2, false>,
                        (const void *)cb_bp_scatter<2, true>,
+                       (const void *)cb_bp_scatter<3, false>,
+                       (const void *)cb_bp_scatter<3, true>,
                        (const void *)cb_bp_scatter<4, false>,
                        (const void *)cb_bp_scatter<4, true>,
                        (const void *)cb_bp_scatter<6, false>,
                        (const void *)cb_bp_scatter<6, true>,
                        (const void *)cb_bp_scatter<8, false>,
-                       (const void *)cb_bp_scatter<8, true>};
+                       (const void *)cb_bp_scatter<8, true>,
+                       (const void *)cb_bp_scatter<10, false>,
+                       (const void *)cb_bp_scatter<10, true>};
 #undef CB_FP_ALL
   for (const void *f : fps)
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, fp) != cudaSuccess)
