@@ -94,7 +94,7 @@ def load_traffic(kernel):
     """DRAM bytes per launch of `kernel` on the full-size workload, from one
     ncu capture of the same command (1-pass metrics), kept in profiles/."""
     name = {"pb_fp": "pb_traffic_768x768x256.json", "pb_bp": "pb_traffic_768x768x256.json",
-            "cb_bp_gather": "cb_traffic_512cube.json", "cb_bp_scatter": "cb_traffic_512cube.json",
+            "cb_bp_tile": "cb_traffic_512cube.json", "cb_bp_scatter": "cb_traffic_512cube.json",
             "cb_fp": "cb_traffic_512cube.json"}.get(kernel)
     if name is None or (kernel.startswith("pb") and globals().get("NH") != 768):
         return None
@@ -116,7 +116,7 @@ def pick_cone_bp(plan, choice):
     else:
         scatter = choice == "scatter"
         plan.set_cone_backprojector(1 if scatter else 0)
-    return ("cb_bp_scatter" if scatter else "cb_bp_gather"), t
+    return ("cb_bp_scatter" if scatter else "cb_bp_tile"), t
 
 
 def load_peaks():

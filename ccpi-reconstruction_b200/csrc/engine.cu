@@ -361,7 +361,8 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     g.inv = inv;
     // one CTA per four rays (a warp each) for the forward projector and the
     // scatter: with 8 CTAs per SM looping over the rays, SMs sat idle at the
-    // end of a launch (512^3: forward 334 -> 306 ms, scatter 629 -> 518 ms);
+    // end of a launch (512^3: forward 334 -> 306 ms, scatter 629 -> 518 ms, in
+    // their forms then);
     // capped so that the FP64 partial sums stay few on huge ray counts
     p->fp_grid = int(std::min<i64>((i64(na) * nh + 3) / 4, i64(sm_count()) * 1024));
     p->bp_parts = cb_bp_parts(g);
@@ -406,7 +407,7 @@ int set_cone_backprojector(ccpi_plan *p, int scatter) {
     return 1;
   }
   p->g.tune_scatter = scatter ? 1 : 0;
-  // one FP64 partial sum per back-projector CTA (gather: one per column),
+  // one FP64 partial sum per back-projector CTA,
   // or per block of the sum-of-squares pass after the scatter
   p->bp_parts = scatter ? sumsq_blocks() : cb_bp_parts(p->g);
   return 0;
