@@ -1046,6 +1046,9 @@ bool pb_fp_one_ray(const Geom &g) {
 struct GroupShape {
   int vec, g, nq, slices;
 };
+size_t group_smem(const Geom &g, int lanes) {
+  return size_t(kLaneWarps) * group_words(32 / lanes, pb_block_room(g)) * 4;
+}
 GroupShape group_shape(const Geom &g) {
   GroupShape s;
   s.slices = g.map_type == 1 ? std::min(g.nv, g.nz) : g.nz;
@@ -1053,10 +1056,10 @@ GroupShape group_shape(const Geom &g) {
   const int lanes = (s.slices + s.vec - 1) / s.vec;
   s.g = lanes <= 4 && s.vec == 4 ? 4 : lanes <= 8 && s.vec == 4 ? 8 : lanes <= 16 ? 16 : 32;
   s.nq = lanes <= 32 ? 1 : lanes <= 64 || s.vec == 4 ? 2 : 4;
+  // very wide grids: fewer rays per warp, whose block lists then fit
+  while (s.g < 32 && group_smem(g, s.g) > 200 * 1024)
+    s.g *= 2;
   return s;
-}
-size_t group_smem(const Geom &g, int lanes) {
-  return size_t(kLaneWarps) * group_words(32 / lanes, pb_block_room(g)) * 4;
 }
 
 template <int EPI>
