@@ -485,7 +485,14 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 2)
   const int2 band = col >= 0 ? g.colband[col] : make_int2(0, 0);
   const float bx = float(g.size[0]), by = float(g.size[1]);
   const float clf = float(g.cl), hscale = float(g.cl * g.cipix), hofs = float(g.chpix0);
-  const float hmargin = 0.02f + 4e-6f * float(g.nh);
+  // A column's candidate rays.  The float projections hl, hh of its corners
+  // are within hround (columns) of the reference's doubles, whose range is
+  // floor(min) .. floor(max) of the columns' even spacing (cb_column_hrange).
+  // With every column within 0.01 of that spacing (even_cols) a ray hmargin
+  // below hl misses the voxel column, and one below hh - hround is in the
+  // range; one between that and hh + hmargin is put to the reference's own
+  // range if it crosses.  Other detectors take that range for every column.
+  const float hround = 4e-6f * float(g.nh), hmargin = 0.02f + hround;
   const double eps = double(kEps);
   const int kb = int(g.pzbz); // every row above the source has k >= kb, every other k <= kb
 
@@ -599,20 +606,21 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 2)
         }
         const double c = g.cosA[a], s = g.sinA[a];
         const double p1x = g.p1x[a], p1y = g.p1y[a];
-        // ---- the column's candidate rays: detector columns between the
-        // projections of its corners, a little widened; the exact test
-        // below decides
+        // ---- the column's candidate rays; the exact tests below decide
         int hA = 0, cnt = 0, rays = 0;
+        float hin = INFINITY; // candidates up to here are in the reference's range
         if (has) {
           float hl, hh, tl, th;
           project_square(float(c * x0 + s * y0 - g.src[0]), float(c * y0 - s * x0 - g.src[1]),
                          float(c), float(s), bx, by, hscale, hofs, hl, hh, tl, th);
           int hB;
-          if (tl > 1e-3f * clf) {
+          if (g.even_cols && tl > 1e-3f * clf) {
+            hin = hh - hround;
             hA = int(fminf(fmaxf(ceilf(hl - hmargin), 0.0f), float(g.nh)));
             hB = int(fmaxf(fminf(floorf(hh + hmargin), float(g.nh - 1)), -1.0f));
           } else {
-            cb_column_hrange(g, a, x0, xn, y0, yn, hA, hB); // beside the source
+            // uneven columns, or beside the source
+            cb_column_hrange(g, a, x0, xn, y0, yn, hA, hB);
           }
           cnt = max(hB - hA + 1, 0);
         }
@@ -633,9 +641,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 2)
             ok = amin < amax - eps;
             a0 = float(amin);
             a1 = float(amax);
-            if (ok && fmax(fabs(inv.x), fabs(inv.y)) * g.cl > 1e6) {
-              // nearly parallel to an axis: rounding may pass a ray that
-              // misses the column, which the reference's range excludes
+            if (ok && (float(h) > hin || fmax(fabs(inv.x), fabs(inv.y)) * g.cl > 1e6)) {
+              // at the range's end, or nearly parallel to an axis, where
+              // rounding may pass a ray that misses the column
               int hmin, hmax;
               cb_column_hrange(g, a, x0, xn, y0, yn, hmin, hmax);
               ok = h >= hmin && h <= hmax;

@@ -52,6 +52,8 @@ struct Geom {
   int mid;                // first row above the source
   float dz0, inv_pitch, pitch_max; // dz[0], 1 / mean row step, largest row step
   int even_rows;          // every row within a quarter step of dz0 + v / inv_pitch
+  int even_cols;          // every column within 0.01 steps of its place in the even
+                          // spacing hpix[0], hpix[1] (cipix), which the axis is near
   const double2 *inv;     // na * nh: 1 / the ray's x and y spans (x = 0: the back
                           // projector takes no such ray, c2D.cpp:909-912)
   float neg0;             // -0.0f (see mul2_nz)

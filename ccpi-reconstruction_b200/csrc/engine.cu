@@ -300,8 +300,14 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
       g.pitch_max = std::max(g.pitch_max, 1.0001f * (dz[i] - dz[i - 1]));
     g.even_rows = 1;
     for (int i = 0; i < nv; i++)
-      if (std::abs((double(dz[i]) - g.dz0) * g.inv_pitch - i) > 0.25)
+      if (!(std::abs((double(dz[i]) - g.dz0) * g.inv_pitch - i) <= 0.25))
         g.even_rows = 0;
+    // the tiled back projector's float estimate of a column's rays holds for
+    // such detectors alone (cb_bp_tile)
+    g.even_cols = nh <= 32768 && std::abs(g.chpix0) <= 4.0 * nh;
+    for (int i = 0; i < nh; i++)
+      if (!(std::abs((hp[i] - hp[0]) * g.cipix - i) <= 0.01))
+        g.even_cols = 0;
     tables.add(g.dconv, dconv);
     tables.add(g.dz, dz);
     tables.add(g.iz, iz);
