@@ -237,7 +237,7 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     tables.add(g.vhi, vhi);
     ok = tables.finish(p);
     p->fp_grid = pb_fp_ctas(g);
-    ok = ok && pb_prepare(g) == 0;
+    ok = ok && pb_prepare() == 0;
     p->bp_parts = pb_bp_tiles(g);
   } else {
     if (nv < 2) {

@@ -33,6 +33,7 @@
 namespace ccpi {
 namespace {
 
+constexpr int kGroupSmem = 200 * 1024; // most shared memory of a pb_fp_groups CTA
 constexpr int kBlock = 32; // the reference's xy block edge (p2D.cpp:498-499)
 
 // std::max / std::min semantics (first argument on ties).
@@ -138,21 +139,28 @@ constexpr int kLaneWarps = 4;
 constexpr int kWalkLanes = PB_WALK_LANES; // blocks walked in parallel per round
 constexpr int kSlotCap = 66;    // cells of one ray in one block (<= 65); even, so
                                 // every other entry starts a 16-byte pair
-constexpr int kMaxBlocks = 192; // blocks one ray may visit (about nbx + nby)
 
 // One staged cell: .x = the column's offset in float4 units (column * nz / 4),
 // .y = the bits of its float length.  Cells outside the volume are dropped
 // when staged (they add nothing).
-struct LaneSmem {
-  uint2 cell[kWalkLanes * kSlotCap];
-  int blk[kMaxBlocks];
-};
+// Words of a warp's staging: its slots, then its block list (room entries).
+constexpr int kLaneGrid = 176;                // nbx + nby at most
+constexpr int kLaneRoom = 2 * kLaneGrid + 8;  // and the list that follows
+__host__ __device__ inline int lane_words(int room) {
+  return (kWalkLanes * kSlotCap * 2 + room + 3) & ~3;
+}
 
 // Blocks of ray (c, s, p2) passing the reference's tests, counted (emit ==
-// nullptr) or written in y-block order for one block column.
+// nullptr) or written in y-block order for one block column: its first is
+// entry pos (below zero: of an earlier list) of a list of room entries
+// (x block << shift | y block).
+//
+// Most rays visit about nbx + nby blocks, but the tests are wide
+// (pb_block_room).
 __device__ __forceinline__ int pb_column_blocks(const Geom &g, int h, double c, double s,
                                                 double p2x, double p2y, bool par_y, bool par_x,
-                                                int bxi, int *emit, int pos, int room) {
+                                                int bxi, int *emit, int pos, int room,
+                                                int shift) {
   const double dx = g.size[0], dy = g.size[1];
   const int nby = (g.ny + kBlock - 1) / kBlock;
   const int bx0 = bxi * kBlock, nxb = min(kBlock, g.nx - bx0);
@@ -190,8 +198,8 @@ __device__ __forceinline__ int pb_column_blocks(const Geom &g, int h, double c, 
       if (jy < 0 || jy >= nyb)
         continue;
     }
-    if (emit && pos + cnt < room)
-      emit[pos + cnt] = (bxi << 16) | byi;
+    if (emit && unsigned(pos + cnt) < unsigned(room))
+      emit[pos + cnt] = (bxi << shift) | byi;
     cnt++;
   }
   return cnt;
@@ -222,19 +230,19 @@ struct RayWalk {
         x_face_first(!(sx > 0 && sy < 0)) {}
 };
 
-// Walk ray W through block id = (x block << 16 | y block) from the block's own
+// Walk ray W through block id = (x block << shift | y block) from the block's own
 // entry point (p2D.cpp:284-458), calling put(column, length) per cell, which
 // counts the cells it keeps in n.  column = gx * ny + gy, formed beyond the
 // volume's edge as the reference forms it.  Returns false if n reached the
 // slot's size before the ray left the block.
 template <class F>
-__device__ __forceinline__ bool pb_walk_slot(const Geom &g, const RayWalk &W, int id, int &n,
-                                             F &&put) {
+__device__ __forceinline__ bool pb_walk_slot(const Geom &g, const RayWalk &W, int id, int shift,
+                                             int &n, F &&put) {
   const double eps = double(kEps);
   const double dx = g.size[0], dy = g.size[1];
   const double c = W.c, s = W.s, p2x = W.p2x, p2y = W.p2y, ic = W.ic, is = W.is;
   const int sx = W.sx, sy = W.sy, ox = sx > 0 ? 1 : 0, oy = sy > 0 ? 1 : 0;
-  const int bxi = id >> 16, byi = id & 0xffff;
+  const int bxi = id >> shift, byi = id & ((1 << shift) - 1);
   const int bx0 = bxi * kBlock, nxb = min(kBlock, g.nx - bx0);
   const int by0 = byi * kBlock, nyb = min(kBlock, g.ny - by0);
   const double vx = g.origin[0] + double(bx0) * dx;
@@ -322,10 +330,12 @@ __device__ __forceinline__ bool pb_walk_slot(const Geom &g, const RayWalk &W, in
 template <int NQ, int EPI>
 __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
     pb_fp_lanes(Geom g, const float *__restrict__ vol, float *__restrict__ pix, Epi e, int v0,
-                int *err) {
+                int room, int *err) {
   extern __shared__ unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  LaneSmem &S = reinterpret_cast<LaneSmem *>(smem_raw)[wib];
+  uint2 *cells = reinterpret_cast<uint2 *>(reinterpret_cast<int *>(smem_raw) +
+                                           wib * lane_words(room));
+  int *blk = reinterpret_cast<int *>(cells + kWalkLanes * kSlotCap);
   const double eps = double(kEps);
   const double dx = g.size[0], dy = g.size[1];
   const int nbx = (g.nx + kBlock - 1) / kBlock;
@@ -372,7 +382,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
       for (int bbase = 0; bbase < nbx; bbase += 32) {
         const int bxi = bbase + lane;
         const int cnt =
-            bxi < nbx ? pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, nullptr, 0, 0)
+            bxi < nbx ? pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, nullptr, 0, 0,
+                                       16)
                     : 0;
         int incl = cnt;
         for (int o = 1; o < 32; o <<= 1) {
@@ -381,14 +392,14 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
             incl += y;
         }
         if (cnt)
-          pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, S.blk, nblk + incl - cnt,
-                           kMaxBlocks);
+          pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, blk, nblk + incl - cnt, room,
+                           16);
         nblk += __shfl_sync(0xffffffffu, incl, 31);
       }
-      if (nblk > kMaxBlocks) {
+      if (nblk > room) {
         if (lane == 0)
           atomicExch(err, 3);
-        nblk = kMaxBlocks;
+        nblk = room;
       }
       __syncwarp();
       const double ic = par_y ? 0.0 : 1.0 / c, is = par_x ? 0.0 : 1.0 / s;
@@ -399,14 +410,14 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
       for (int r0 = 0; r0 < nblk; r0 += kWalkLanes) {
         const int j = r0 + lane;
         int n = 0;
-        uint2 *myc = S.cell + (lane % kWalkLanes) * kSlotCap;
+        uint2 *myc = cells + (lane % kWalkLanes) * kSlotCap;
         auto put = [&](int col, float len) {
           if (unsigned(col) < unsigned(ncol))
             myc[n++] = make_uint2(unsigned(col) * nz4, __float_as_uint(len));
         };
         // pb_walk_slot, written out: as a call it costs this kernel 1 % in spills
         if (lane < kWalkLanes && j < nblk) {
-          const int id = S.blk[j];
+          const int id = blk[j];
           const int bxi = id >> 16, byi = id & 0xffff;
           const int bx0 = bxi * kBlock, nxb = min(kBlock, g.nx - bx0);
           const int by0 = byi * kBlock, nyb = min(kBlock, g.ny - by0);
@@ -489,7 +500,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, PB_FP_MINB)
         const int nr = min(kWalkLanes, nblk - r0);
         for (int jj = 0; jj < nr; jj++) {
           const int nj = __shfl_sync(0xffffffffu, n, jj);
-          const uint2 *cl = S.cell + jj * kSlotCap;
+          const uint2 *cl = cells + jj * kSlotCap;
           int m = 0;
 #if PB_FP_BATCH == 4
           for (; m + 4 <= nj; m += 4) {
@@ -592,7 +603,10 @@ __host__ __device__ inline int group_words(int rays, int room) {
   return (32 * kSlotCap * 2 + 32 + rays * room + 3) & ~3;
 }
 
-template <int VEC, int G, int NQ, int EPI>
+// LISTS: the block list of a ray may need several lists, traced one after the
+// other (grids of more than some 130,000 columns along an axis; as a rule for
+// all grids it costs 0 to 5 %).
+template <int VEC, int G, int NQ, int EPI, bool LISTS = false>
 __global__ void __launch_bounds__(kLaneWarps * 32)
     pb_fp_groups(Geom g, const float *__restrict__ vol, float *__restrict__ pix, Epi e, int z0,
                  int room, int *err) {
@@ -608,6 +622,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32)
   const double eps = double(kEps);
   const int nbx = (g.nx + kBlock - 1) / kBlock;
   const int ncol = g.nx * g.ny;
+  const int shift = 32 - __clz((g.ny - 1) / kBlock); // bits of a y block
   const float2 nz2 = make_float2(g.neg0, g.neg0);
   // slices z0 + (q * G + l) * VEC + i
   bool zok[NQ];
@@ -628,12 +643,16 @@ __global__ void __launch_bounds__(kLaneWarps * 32)
     const bool par_y = fabs(c) < eps, par_x = !par_y && fabs(s) < eps;
     const bool some = a < g.na && !(par_y && fabs(s) < eps);
     V acc[NQ] = {};
+    int first = 0; // block that the list starts at
+    bool more;
+    do {
     // ---- the ray's blocks: x-block major, y-block ascending
-    int nblk = 0;
+    int nblk = -first;
     for (int b0 = 0; b0 < nbx; b0 += G) {
       const int bxi = b0 + l;
       const int n = (some && bxi < nbx)
-                        ? pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, nullptr, 0, 0)
+                        ? pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, nullptr, 0, 0,
+                                           shift)
                         : 0;
       int incl = n;
       for (int o = 1; o < G; o <<= 1) {
@@ -642,11 +661,13 @@ __global__ void __launch_bounds__(kLaneWarps * 32)
           incl += y;
       }
       if (n)
-        pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, blk, nblk + incl - n, room);
+        pb_column_blocks(g, h, c, s, p2x, p2y, par_y, par_x, bxi, blk, nblk + incl - n, room,
+                         shift);
       nblk += __shfl_sync(0xffffffffu, incl, G - 1, G);
     }
+    more = LISTS && __any_sync(0xffffffffu, nblk > room);
     if (nblk > room) {
-      if (l == 0)
+      if (!LISTS && l == 0)
         atomicExch(err, 3);
       nblk = room;
     }
@@ -657,7 +678,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32)
       // ---- one block per lane
       uint2 *mine = cells + lane * kSlotCap;
       int n = 0;
-      if (r0 + l < nblk && !pb_walk_slot(g, W, blk[r0 + l], n, [&](int col, float len) {
+      if (r0 + l < nblk && !pb_walk_slot(g, W, blk[r0 + l], shift, n, [&](int col, float len) {
             if (unsigned(col) < unsigned(ncol))
               mine[n++] = make_uint2(unsigned(col), __float_as_uint(len));
           }))
@@ -702,12 +723,15 @@ __global__ void __launch_bounds__(kLaneWarps * 32)
               if (u < left && zok[q])
                 add_cell(acc[q], x[u][q], len[u], nz2);
         }
-        // a group that is done stays where it is: its reads stay in the slots
+        // a group that is done stays where it is; the reads past a slot's last
+        // cell fall in the next slot or, after the last, in the counts
         cl += left > 0 ? 4 : 0;
         left = max(left - 4, 0);
       }
       __syncwarp();
     }
+    first += room;
+    } while (more);
     // ---- store every slice's sum to its rows; rows of no slice are zero
     if (a < g.na) {
       const i64 rbase = (i64(a) * g.nh + h) * g.nv;
@@ -1029,15 +1053,23 @@ __global__ void __launch_bounds__(256) pb_bp_scalar(Geom g, const float *__restr
     store_partial<8>(ssq, e);
 }
 
+// Blocks that a ray lists at most.  pb_column_blocks takes, in every block
+// column, the block rows within 1e-3 voxels of the ray: one, and one more per
+// boundary of block rows that is so close.  A ray that rises by more than that
+// in a block column comes close to a boundary in two columns at most (on a
+// diagonal through block corners it does at every boundary); a flatter one
+// reaches one boundary, in up to all of them.
+int pb_block_room(const Geom &g) {
+  const int nbx = (g.nx + kBlock - 1) / kBlock, nby = (g.ny + kBlock - 1) / kBlock;
+  return nbx + std::max(nbx, 2 * nby) + 8;
+}
 // The one-ray-per-warp kernel applies: row v <-> slice v, float4 rows that
 // fill more than half a warp, float4 offsets of the columns fit 32 bits, and
-// a ray's block list (at most about nbx + nby entries) fits its staging area.
-int pb_block_room(const Geom &g) {
-  return (g.nx + kBlock - 1) / kBlock + (g.ny + kBlock - 1) / kBlock + 16;
-}
+// the grid is not so wide that the block lists keep CTAs off an SM.
 bool pb_fp_one_ray(const Geom &g) {
   return g.map_type == 1 && (g.nv % 4) == 0 && (g.nz % 4) == 0 && g.nv > 64 &&
-         (long long)g.nx * g.ny * (g.nz / 4) < (1ll << 32) && pb_block_room(g) <= kMaxBlocks;
+         (long long)g.nx * g.ny * (g.nz / 4) < (1ll << 32) &&
+         (g.nx + kBlock - 1) / kBlock + (g.ny + kBlock - 1) / kBlock <= kLaneGrid;
 }
 
 // Lanes per ray and slices per lane for the others: the fewest lanes that
@@ -1045,10 +1077,10 @@ bool pb_fp_one_ray(const Geom &g) {
 // 2 float4 or 4 floats per lane and launch.
 struct GroupShape {
   int vec, g, nq, slices;
+  bool lists; // rays with more blocks than room take list after list
+  int room;
+  size_t smem;
 };
-size_t group_smem(const Geom &g, int lanes) {
-  return size_t(kLaneWarps) * group_words(32 / lanes, pb_block_room(g)) * 4;
-}
 GroupShape group_shape(const Geom &g) {
   GroupShape s;
   s.slices = g.map_type == 1 ? std::min(g.nv, g.nz) : g.nz;
@@ -1056,9 +1088,17 @@ GroupShape group_shape(const Geom &g) {
   const int lanes = (s.slices + s.vec - 1) / s.vec;
   s.g = lanes <= 4 && s.vec == 4 ? 4 : lanes <= 8 && s.vec == 4 ? 8 : lanes <= 16 ? 16 : 32;
   s.nq = lanes <= 32 ? 1 : lanes <= 64 || s.vec == 4 ? 2 : 4;
+  s.room = pb_block_room(g);
+  auto smem = [&] { return size_t(kLaneWarps) * group_words(32 / s.g, s.room) * 4; };
   // very wide grids: fewer rays per warp, whose block lists then fit
-  while (s.g < 32 && group_smem(g, s.g) > 200 * 1024)
+  while (s.g < 32 && smem() > kGroupSmem)
     s.g *= 2;
+  s.lists = smem() > kGroupSmem;
+  if (s.lists) {
+    s.nq = 1;
+    s.room = 2048; // two CTAs per SM
+  }
+  s.smem = smem();
   return s;
 }
 
@@ -1066,22 +1106,27 @@ template <int EPI>
 int launch_fp(const Geom &g, const float *vol, float *pix, const Epi &e, int grid, int *err,
               cudaStream_t st) {
   if (pb_fp_one_ray(g)) {
-    const size_t smem = sizeof(LaneSmem) * kLaneWarps;
+    const int room = pb_block_room(g);
+    const size_t smem = size_t(kLaneWarps) * lane_words(room) * 4;
     for (int v0 = 0; v0 < g.nv; v0 += 256) {
       if (g.nv - v0 > 128)
-        pb_fp_lanes<2, EPI><<<grid, kLaneWarps * 32, smem, st>>>(g, vol, pix, e, v0, err);
+        pb_fp_lanes<2, EPI><<<grid, kLaneWarps * 32, smem, st>>>(g, vol, pix, e, v0, room, err);
       else
-        pb_fp_lanes<1, EPI><<<grid, kLaneWarps * 32, smem, st>>>(g, vol, pix, e, v0, err);
+        pb_fp_lanes<1, EPI><<<grid, kLaneWarps * 32, smem, st>>>(g, vol, pix, e, v0, room, err);
     }
     return 0;
   }
   const GroupShape s = group_shape(g);
-  const size_t smem = group_smem(g, s.g);
-  const int room = pb_block_room(g);
   for (int z0 = 0; z0 < s.slices; z0 += s.g * s.nq * s.vec) {
-#define PB_GROUPS(V, L, Q)                                                                 \
-  pb_fp_groups<V, L, Q, EPI><<<grid, kLaneWarps * 32, smem, st>>>(g, vol, pix, e, z0, room, err)
-    if (s.vec == 4) {
+#define PB_GROUPS(V, L, Q, ...)                                                            \
+  pb_fp_groups<V, L, Q, EPI, ##__VA_ARGS__><<<grid, kLaneWarps * 32, s.smem, st>>>(          \
+      g, vol, pix, e, z0, s.room, err)
+    if (s.lists) {
+      if (s.vec == 4)
+        PB_GROUPS(4, 32, 1, true);
+      else
+        PB_GROUPS(1, 32, 1, true);
+    } else if (s.vec == 4) {
       if (s.g == 4)
         PB_GROUPS(4, 4, 1);
       else if (s.g == 8)
@@ -1212,9 +1257,7 @@ int pb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi 
 
 // Opt the forward kernels into their shared memory (done once, outside any
 // graph capture).
-int pb_prepare(const Geom &g) {
-  if (group_smem(g, group_shape(g).g) > 200 * 1024)
-    return 1;
+int pb_prepare() {
   bool ok = true;
   auto allow = [&](const void *f, int smem) {
     ok = ok &&
@@ -1223,14 +1266,16 @@ int pb_prepare(const Geom &g) {
 #define PB_ALL(E)                                                                          \
   {                                                                                        \
     for (const void *f : {(const void *)pb_fp_lanes<1, E>, (const void *)pb_fp_lanes<2, E>}) \
-      allow(f, int(sizeof(LaneSmem) * kLaneWarps));                                         \
+      allow(f, kLaneWarps * lane_words(kLaneRoom) * 4);                                        \
     for (const void *f :                                                                    \
          {(const void *)pb_fp_groups<4, 4, 1, E>, (const void *)pb_fp_groups<4, 8, 1, E>,    \
           (const void *)pb_fp_groups<4, 16, 1, E>, (const void *)pb_fp_groups<4, 32, 1, E>,  \
           (const void *)pb_fp_groups<4, 32, 2, E>, (const void *)pb_fp_groups<1, 16, 1, E>,  \
           (const void *)pb_fp_groups<1, 32, 1, E>, (const void *)pb_fp_groups<1, 32, 2, E>,  \
-          (const void *)pb_fp_groups<1, 32, 4, E>})                                          \
-      allow(f, 200 * 1024);                                                                 \
+          (const void *)pb_fp_groups<1, 32, 4, E>,                                           \
+          (const void *)pb_fp_groups<4, 32, 1, E, true>,                                     \
+          (const void *)pb_fp_groups<1, 32, 1, E, true>})                                    \
+      allow(f, kGroupSmem);                                                                 \
   }
   PB_ALL(EPI_STORE)
   PB_ALL(EPI_NORM)
