@@ -1063,18 +1063,26 @@ int pb_block_room(const Geom &g) {
   const int nbx = (g.nx + kBlock - 1) / kBlock, nby = (g.ny + kBlock - 1) / kBlock;
   return nbx + std::max(nbx, 2 * nby) + 8;
 }
-// The one-ray-per-warp kernel applies: row v <-> slice v, float4 rows that
-// fill more than half a warp, float4 offsets of the columns fit 32 bits, and
-// the grid is not so wide that the block lists keep CTAs off an SM.
+// The one-ray-per-warp kernel applies: row v <-> slice v, float4 rows, float4
+// offsets of the columns fit 32 bits, and the grid is not so wide that the
+// block lists keep CTAs off an SM.  It is the faster one where the rows fill
+// more than half a warp, and where so few rays sharing warps would leave the
+// GPU idle.  One ray per warp / shared, us: four lanes per ray, 192^2 x 16,
+// 1,560 rays 45 / 83, 3,900 rays 64 / 82, 5,850 rays 98 / 78; 512^2 x 4, 515 rays 43 /
+// 125, 4,120 rays 128 / 229; more lanes per ray, 192^2 x 24, 2,730 rays 53 / 60,
+// 256^2 x 32, 3,626 rays 80 / 70, 192^2 x 64, 2,925 rays 53 / 49.
 bool pb_fp_one_ray(const Geom &g) {
-  return g.map_type == 1 && (g.nv % 4) == 0 && (g.nz % 4) == 0 && g.nv > 64 &&
+  const i64 rays = i64(g.na) * g.nh;
+  const bool few = rays <= (g.nv > 16 ? 2800 : 4400);
+  return g.map_type == 1 && (g.nv % 4) == 0 && (g.nz % 4) == 0 && (g.nv > 64 || few) &&
          (long long)g.nx * g.ny * (g.nz / 4) < (1ll << 32) &&
          (g.nx + kBlock - 1) / kBlock + (g.ny + kBlock - 1) / kBlock <= kLaneGrid;
 }
 
 // Lanes per ray and slices per lane for the others: the fewest lanes that
 // hold the rows' slices (slices past the last row's need no sum), then up to
-// 2 float4 or 4 floats per lane and launch.
+// 2 float4 or 8 floats per lane and launch (255 slices with 4 floats, in two
+// launches: 64^2, 90 angles 181 us against 120, 192^2 944 against 673).
 struct GroupShape {
   int vec, g, nq, slices;
   bool lists; // rays with more blocks than room take list after list
@@ -1087,7 +1095,7 @@ GroupShape group_shape(const Geom &g) {
   s.vec = g.nz % 4 == 0 ? 4 : 1;
   const int lanes = (s.slices + s.vec - 1) / s.vec;
   s.g = lanes <= 4 && s.vec == 4 ? 4 : lanes <= 8 && s.vec == 4 ? 8 : lanes <= 16 ? 16 : 32;
-  s.nq = lanes <= 32 ? 1 : lanes <= 64 || s.vec == 4 ? 2 : 4;
+  s.nq = lanes <= 32 ? 1 : lanes <= 64 || s.vec == 4 ? 2 : lanes <= 128 ? 4 : 8;
   s.room = pb_block_room(g);
   auto smem = [&] { return size_t(kLaneWarps) * group_words(32 / s.g, s.room) * 4; };
   // very wide grids: fewer rays per warp, whose block lists then fit
@@ -1144,8 +1152,10 @@ int launch_fp(const Geom &g, const float *vol, float *pix, const Epi &e, int gri
         PB_GROUPS(1, 32, 1);
       else if (s.nq == 2)
         PB_GROUPS(1, 32, 2);
-      else
+      else if (s.nq == 4)
         PB_GROUPS(1, 32, 4);
+      else
+        PB_GROUPS(1, 32, 8);
     }
 #undef PB_GROUPS
   }
@@ -1272,7 +1282,7 @@ int pb_prepare() {
           (const void *)pb_fp_groups<4, 16, 1, E>, (const void *)pb_fp_groups<4, 32, 1, E>,  \
           (const void *)pb_fp_groups<4, 32, 2, E>, (const void *)pb_fp_groups<1, 16, 1, E>,  \
           (const void *)pb_fp_groups<1, 32, 1, E>, (const void *)pb_fp_groups<1, 32, 2, E>,  \
-          (const void *)pb_fp_groups<1, 32, 4, E>,                                           \
+          (const void *)pb_fp_groups<1, 32, 4, E>, (const void *)pb_fp_groups<1, 32, 8, E>,  \
           (const void *)pb_fp_groups<4, 32, 1, E, true>,                                     \
           (const void *)pb_fp_groups<1, 32, 1, E, true>})                                    \
       allow(f, kGroupSmem);                                                                 \
