@@ -30,7 +30,6 @@
 #include <climits>
 #include <cmath>
 #include <type_traits>
-#include <utility>
 
 #include "cb_common.cuh"
 #include "kernels.h"
@@ -723,10 +722,10 @@ __global__ void cb_ray_spans_kernel(Geom g, double2 *inv) {
   }
 }
 
-// ---- small volumes: one CTA per column
+// ---- few columns: one CTA per column
 //
 // Too few columns to give every SM a tile of them: one CTA owns one column
-// and each thread one of its voxels.  Rays are staged per angle chunk.  For a
+// and each thread up to four of its voxels and rows.  Rays are staged per angle chunk.  For a
 // stage of ST rays each thread loads its band rows (RMAX per ray, all loads in
 // flight together), forms every row's two contributions and records, for
 // every slice K, the first band row whose index reaches K (k is monotone in
@@ -814,9 +813,10 @@ __device__ __forceinline__ void cb_ga_mark(int *f, int kp, int k, int v, int nz)
 
 // PRE: the sinogram is already scaled by d_conv (the reference's dpixels,
 // c2D.cpp:1096-1117), so a staged row is one load and no multiply.  ST rays
-// per stage.  T threads, one per voxel.  blockIdx.y: the sinogram of a batch.
-template <int EPI, int T, int RMAX, bool PRE, int ST>
-__global__ void __launch_bounds__(T, 1024 / T)
+// per stage.  T threads, each with NZT voxels and RMAX rows.  blockIdx.y: the
+// sinogram of a batch.
+template <int EPI, int T, int NZT, int RMAX, bool PRE, int ST>
+__global__ void __launch_bounds__(T, NZT == 1 ? 1024 / T : NZT == 2 ? 3 : 2)
     cb_bp_column(Geom g, const float *__restrict__ pix0, float *__restrict__ vol0, Epi e,
                  int *err) {
   extern __shared__ unsigned char smem_raw[];
@@ -881,8 +881,10 @@ __global__ void __launch_bounds__(T, 1024 / T)
   double ssq = 0.0;
   const float *__restrict__ pix = pix0 + i64(blockIdx.y) * g.na * g.nh * nv;
   float *__restrict__ vol = vol0 + i64(blockIdx.y) * g.nx * g.ny * nz;
-  const int K = tid; // this thread's voxel
-  float acc = 0.0f;
+  float acc[NZT]; // this thread's voxels tid + z * T
+#pragma unroll
+  for (int z = 0; z < NZT; z++)
+    acc[z] = 0.0f;
 
   // ---- band rows of every ray (c2D.cpp:680-713)
   for (int ac = 0; nb > 0 && ac < g.na; ac += kGaChunk) {
@@ -998,19 +1000,23 @@ __global__ void __launch_bounds__(T, 1024 / T)
         const int *f = fr + s * frs;
         const float *c1 = prow + s * prs, *c2 = drow + s * prs;
         const int klo = s_kf[s] - 1, khi = s_kl[s] + 1;
-        if (K >= nz || K < klo || K > khi)
-          continue; // no row of this ray feeds voxel K
-        const int fm = K >= 1 ? f[K - 1] : min_v, f0 = f[K], f1 = f[K + 1];
-        float t = acc;
-        // below the source row: rows of slice K give c1, then rows of
-        // slice K + 1 give c2 (their neighbour k - 1 == K)
-        for (int v = f0, ve = min(f[K + 2], lo_end); v < ve; v++)
-          t = __fadd_rn(t, (v < f1 ? c1 : c2)[v]);
-        // from the source row on: rows of slice K - 1 give c2 (their
-        // neighbour k + 1 == K), then rows of slice K give c1
-        for (int v = max(fm, up_begin), ve = min(f1, max_v); v < ve; v++)
-          t = __fadd_rn(t, (v < f0 ? c2 : c1)[v]);
-        acc = t;
+#pragma unroll
+        for (int z = 0; z < NZT; z++) {
+          const int K = tid + z * T;
+          if (K >= nz || K < klo || K > khi)
+            continue; // no row of this ray feeds voxel K
+          const int fm = K >= 1 ? f[K - 1] : min_v, f0 = f[K], f1 = f[K + 1];
+          float t = acc[z];
+          // below the source row: rows of slice K give c1, then rows of
+          // slice K + 1 give c2 (their neighbour k - 1 == K)
+          for (int v = f0, ve = min(f[K + 2], lo_end); v < ve; v++)
+            t = __fadd_rn(t, (v < f1 ? c1 : c2)[v]);
+          // from the source row on: rows of slice K - 1 give c2 (their
+          // neighbour k + 1 == K), then rows of slice K give c1
+          for (int v = max(fm, up_begin), ve = min(f1, max_v); v < ve; v++)
+            t = __fadd_rn(t, (v < f0 ? c2 : c1)[v]);
+          acc[z] = t;
+        }
       }
       __syncthreads();
     }
@@ -1029,44 +1035,52 @@ __global__ void __launch_bounds__(T, 1024 / T)
         const float av = __fmul_rn(a0, inv_dz);
         const float *prw = pix + (i64(ac + m / kGaRays) * g.nh + h) * nv;
         const float *drw = g.dconv + i64(h) * nv;
-        if (K >= nz)
-          continue;
-        for (int v = min(min_v, nv) - 1; v >= 0; v--) {
-          const int k = int(__fadd_rn(pzbz1, __fmul_rn(av, sdz[v]))) - 1;
-          if (k < K)
-            break; // k only falls as v falls (and k < 0 ends the reference's loop)
-          if (k > K + 1)
+#pragma unroll
+        for (int z = 0; z < NZT; z++) {
+          const int K = tid + z * T;
+          if (K >= nz)
             continue;
-          const float p = PRE ? __ldg(prw + v) : __fmul_rn(__ldg(prw + v), __ldg(drw + v));
-          if (k > 0) {
-            const float mz = fmin_ref(__fmul_rn(svz[k], siz[v]), a1);
-            acc = __fadd_rn(acc, __fmul_rn(p, k == K ? __fsub_rn(mz, a0)
-                                                           : __fsub_rn(a1, mz)));
-          } else if (K == 0) {
-            const float mz = fmin_ref(__fmul_rn(svz[0], siz[v]), a1);
-            acc = __fadd_rn(acc, __fmul_rn(p, __fsub_rn(mz, a0)));
+          for (int v = min(min_v, nv) - 1; v >= 0; v--) {
+            const int k = int(__fadd_rn(pzbz1, __fmul_rn(av, sdz[v]))) - 1;
+            if (k < K)
+              break; // k only falls as v falls (and k < 0 ends the reference's loop)
+            if (k > K + 1)
+              continue;
+            const float p = PRE ? __ldg(prw + v) : __fmul_rn(__ldg(prw + v), __ldg(drw + v));
+            if (k > 0) {
+              const float mz = fmin_ref(__fmul_rn(svz[k], siz[v]), a1);
+              acc[z] = __fadd_rn(acc[z], __fmul_rn(p, k == K ? __fsub_rn(mz, a0)
+                                                             : __fsub_rn(a1, mz)));
+            } else if (K == 0) {
+              const float mz = fmin_ref(__fmul_rn(svz[0], siz[v]), a1);
+              acc[z] = __fadd_rn(acc[z], __fmul_rn(p, __fsub_rn(mz, a0)));
+            }
           }
-        }
-        for (int v = max(max_v, 0); v < nv; v++) {
-          const int k = int(__fadd_rn(pzbz, __fmul_rn(av, sdz[v])));
-          if (k > K || k > nzm1)
-            break; // k only rises with v (and k > nz - 1 ends the reference's loop)
-          if (k < K - 1)
-            continue;
-          const float p = PRE ? __ldg(prw + v) : __fmul_rn(__ldg(prw + v), __ldg(drw + v));
-          const float mz = fmin_ref(__fmul_rn(svz[k + 1], siz[v]), a1);
-          if (k == K)
-            acc = __fadd_rn(acc, __fmul_rn(p, __fsub_rn(mz, a0)));
-          else if (k < nzm1)
-            acc = __fadd_rn(acc, __fmul_rn(p, __fsub_rn(a1, mz)));
+          for (int v = max(max_v, 0); v < nv; v++) {
+            const int k = int(__fadd_rn(pzbz, __fmul_rn(av, sdz[v])));
+            if (k > K || k > nzm1)
+              break; // k only rises with v (and k > nz - 1 ends the reference's loop)
+            if (k < K - 1)
+              continue;
+            const float p = PRE ? __ldg(prw + v) : __fmul_rn(__ldg(prw + v), __ldg(drw + v));
+            const float mz = fmin_ref(__fmul_rn(svz[k + 1], siz[v]), a1);
+            if (k == K)
+              acc[z] = __fadd_rn(acc[z], __fmul_rn(p, __fsub_rn(mz, a0)));
+            else if (k < nzm1)
+              acc[z] = __fadd_rn(acc[z], __fmul_rn(p, __fsub_rn(a1, mz)));
+          }
         }
       }
       __syncthreads();
     }
   }
   const i64 base = i64(col) * nz;
-  if (K < nz) {
-    const float v = acc;
+#pragma unroll
+  for (int z = 0; z < NZT; z++) {
+    const int K = tid + z * T;
+    if (K >= nz)
+      break;
+    const float v = acc[z];
     float o = v;
     if (EPI == EPI_NORM) {
       ssq += double(v) * double(v);
@@ -1089,22 +1103,30 @@ __global__ void __launch_bounds__(T, 1024 / T)
   }
 }
 
-// Which kernel: the tiles need some 2,000 warps of 32 columns x 8 or more
-// slices to fill the GPU; below that a CTA per column wins.  Cubes with the
-// 512^3 benchmark's proportions, column / tile kernel: 48^3 0.41 / 0.80 ms,
-// 64^3 0.84 / 1.45, 80^3 1.70 / 2.16, 96^3 3.47 / 2.62, 128^3 7.75 / 7.17.
-// The column kernel holds one voxel and two rows per thread.
+// Which kernel: a CTA per column costs its columns' rays and rows; the tiles'
+// time is flat until there are columns enough for every SM.  Column / tile
+// kernel, cubes with the 512^3 benchmark's proportions, 90 angles: 48^3 0.41 /
+// 0.80 ms, 64^3 0.84 / 1.45, 80^3 1.70 / 2.16, 96^3 3.47 / 2.62; with two rays
+// and two rows per voxel the tiles win from 64^3 (0.55 / 0.41 ms, 24 angles).
+// On few columns the tiles lose at any height and row count: 32^2 x 512 from
+// 768 rows 388 / 457 us, x 64 from 520 600 / 1190, 40^2 x 512 from 256 355 /
+// 364, but 40^2 x 900 from 450 586 / 489.
 bool small_volume(const Geom &g) {
-  return i64(g.nx) * g.ny * g.nz <= (1 << 19) && g.nz <= 256 && g.nv <= 512;
+  const i64 columns = i64(g.nx) * g.ny, voxels = columns * g.nz;
+  return g.nz <= 1024 && g.nv <= 1024 &&
+         ((voxels <= (1 << 19) && g.nz <= 256 && g.nv <= 512) ||
+          (columns <= 1600 && voxels <= (1 << 20)));
 }
 
 size_t small_smem(const Geom &g) {
   return size_t(GaLayout(g.nz, g.nv, std::max(kGaStage, kGaStagePre)).total) * 4;
 }
 
-// Chunk height and warps per CTA.  Tall chunks spend less on ray set-up and
-// on rows that straddle two chunks; small problems need short chunks and
-// small CTAs to reach every SM.  32 slices, 8 warps and 17,000 patch floats
+// Chunk height; warps per CTA.  Tall chunks spend less on ray set-up and
+// on rows that straddle two chunks; small problems need short chunks to reach
+// every SM.  Eight warps share a patch: CTAs of two or four, which would reach
+// more SMs, spend more on the copies (64^3 from 96 rows, 24 angles: 406 us, with two
+// warps 766).  32 slices, 8 warps and 17,000 patch floats
 // make two CTAs per SM (36 KB of accumulators, 4 KB of row tables and 66 KB
 // of patch each); 512^3: 617 ms, 660 ms with 24 slices, 831 ms with 16 slices
 // and three CTAs, 676 ms with one CTA of 16 warps.
@@ -1117,8 +1139,6 @@ TileShape tile_shape(const Geom &g) {
   t.nzc = (g.nz + t.zc - 1) / t.zc;
   t.wx = 2;
   t.wy = 4;
-  while (t.wy > 1 && warps * t.nzc < i64(296) * t.wx * t.wy)
-    t.wy /= 2;
   t.rcap = 512;
   t.cap = 17000;
   t.ntx = (g.nx + t.wx * kTileX - 1) / (t.wx * kTileX);
@@ -1126,17 +1146,21 @@ TileShape tile_shape(const Geom &g) {
   return t;
 }
 
-template <int EPI, bool PRE>
-void launch_small(const Geom &g, dim3 grid, const float *pix, float *vol, const Epi &e, int *err,
-                  cudaStream_t st) {
+// The column kernel's instance for a plan's slices and rows; its threads.
+typedef void (*ColumnKernel)(Geom, const float *, float *, Epi, int *);
+int column_threads(const Geom &g) { return g.nz <= 128 && g.nv <= 256 ? 128 : 256; }
+template <int EPI, bool PRE> ColumnKernel column_kernel(const Geom &g) {
   constexpr int ST = PRE ? kGaStagePre : kGaStage;
-  const size_t smem = small_smem(g);
-  if (g.nz <= 128 && g.nv <= 128)
-    cb_bp_column<EPI, 128, 1, PRE, ST><<<grid, 128, smem, st>>>(g, pix, vol, e, err);
-  else if (g.nz <= 128 && g.nv <= 256)
-    cb_bp_column<EPI, 128, 2, PRE, ST><<<grid, 128, smem, st>>>(g, pix, vol, e, err);
-  else
-    cb_bp_column<EPI, 256, 2, PRE, ST><<<grid, 256, smem, st>>>(g, pix, vol, e, err);
+#define CB_COLUMN_ROWS(Z)                                                                  \
+  (g.nv <= 256   ? cb_bp_column<EPI, 256, Z, 1, PRE, ST>                                    \
+   : g.nv <= 512 ? cb_bp_column<EPI, 256, Z, 2, PRE, ST>                                    \
+   : g.nv <= 768 ? cb_bp_column<EPI, 256, Z, 3, PRE, ST>                                    \
+                 : cb_bp_column<EPI, 256, Z, 4, PRE, ST>)
+  if (column_threads(g) == 128)
+    return g.nv <= 128 ? cb_bp_column<EPI, 128, 1, 1, PRE, ST>
+                       : cb_bp_column<EPI, 128, 1, 2, PRE, ST>;
+  return g.nz <= 256 ? CB_COLUMN_ROWS(1) : g.nz <= 512 ? CB_COLUMN_ROWS(2) : CB_COLUMN_ROWS(4);
+#undef CB_COLUMN_ROWS
 }
 
 template <int EPI>
@@ -1146,11 +1170,10 @@ void launch_bp(const Geom &g, const float *pix, float *vol, const Epi &e, int *e
   const TileShape t = tile_shape(g);
   for (int b = 0; b < nbatch; b += 65535) {
     const unsigned ny = std::min(nbatch - b, 65535);
-    if (small_volume(g) && e.pre)
-      launch_small<EPI, true>(g, dim3(g.nx * g.ny, ny), pix + b * nin, vol + b * nout, e, err, st);
-    else if (small_volume(g))
-      launch_small<EPI, false>(g, dim3(g.nx * g.ny, ny), pix + b * nin, vol + b * nout, e, err,
-                               st);
+    if (small_volume(g))
+      (e.pre ? column_kernel<EPI, true>(g) : column_kernel<EPI, false>(g))
+          <<<dim3(g.nx * g.ny, ny), column_threads(g), small_smem(g), st>>>(
+              g, pix + b * nin, vol + b * nout, e, err);
     else
       cb_bp_tile<EPI><<<dim3(t.ntx * t.nty * t.nzc, ny), t.wx * t.wy * 32, tile_smem(t), st>>>(
           g, pix + b * nin, vol + b * nout, e, err, t);
@@ -1174,26 +1197,24 @@ int cb_bp_parts(const Geom &g) {
   return small_volume(g) ? g.nx * g.ny : t.ntx * t.nty * t.nzc;
 }
 
-int cb_bp_prepare() {
-#define CB_BP_ALL(F) F(EPI_STORE), F(EPI_NORM), F(EPI_SIRT), F(EPI_MLEM)
-#define CB_TILE(E) (const void *)cb_bp_tile<E>
-#define CB_COLUMN(E)                                                                       \
-  (const void *)cb_bp_column<E, 128, 1, false, kGaStage>,                                   \
-      (const void *)cb_bp_column<E, 128, 2, false, kGaStage>,                               \
-      (const void *)cb_bp_column<E, 256, 2, false, kGaStage>,                               \
-      (const void *)cb_bp_column<E, 128, 1, true, kGaStagePre>,                             \
-      (const void *)cb_bp_column<E, 128, 2, true, kGaStagePre>,                             \
-      (const void *)cb_bp_column<E, 256, 2, true, kGaStagePre>
-  const void *tiles[] = {CB_BP_ALL(CB_TILE)}, *columns[] = {CB_BP_ALL(CB_COLUMN)};
-#undef CB_COLUMN
-#undef CB_TILE
-#undef CB_BP_ALL
+int cb_bp_prepare(const Geom &g) {
   // the limit is the function's, not the plan's: the largest any plan uses
   bool ok = true;
-  for (const auto &list : {std::make_pair(tiles, 4), std::make_pair(columns, 24)})
-    for (int n = 0; n < list.second; n++)
-      ok = ok && cudaFuncSetAttribute(list.first[n], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      220 * 1024) == cudaSuccess;
+  auto allow = [&](const void *f) {
+    ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    220 * 1024) == cudaSuccess;
+  };
+#define CB_BP_ALLOW(E)                                                                     \
+  if (small_volume(g)) {                                                                    \
+    allow((const void *)column_kernel<E, false>(g));                                        \
+    allow((const void *)column_kernel<E, true>(g));                                         \
+  } else                                                                                    \
+    allow((const void *)cb_bp_tile<E>);
+  CB_BP_ALLOW(EPI_STORE)
+  CB_BP_ALLOW(EPI_NORM)
+  CB_BP_ALLOW(EPI_SIRT)
+  CB_BP_ALLOW(EPI_MLEM)
+#undef CB_BP_ALLOW
   return ok ? 0 : 1;
 }
 

@@ -879,7 +879,7 @@ void launch_cb_fp(const Geom &g, const float *vol, float *pix, const Epi &e, con
 }
 } // namespace
 
-int cb_prepare() {
+int cb_prepare(const Geom &g) {
   // the limit is the function's, not the plan's: the largest any plan uses
   const int fp = 200 * 1024;
 #define CB_FP_ALL(R)                                                                       \
@@ -905,7 +905,7 @@ int cb_prepare() {
   for (const void *f : fps)
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, fp) != cudaSuccess)
       return 1;
-  return cb_bp_prepare();
+  return cb_bp_prepare(g);
 }
 
 int cb_forward(const Geom &g, const float *vol, float *pix, int mode, const Epi &e,

@@ -360,7 +360,7 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     double2 *inv = nullptr;
     tables.reserve(band, size_t(g.nx) * g.ny);
     tables.reserve(inv, size_t(na) * nh);
-    ok = cb_prepare() == 0 && tables.finish(p);
+    ok = cb_prepare(g) == 0 && tables.finish(p);
     p->hrange = const_cast<int2 *>(hrange);
     ok = ok && cb_column_bands(g, band, 0) == 0 && cb_ray_spans(g, inv, 0) == 0;
     g.colband = band;

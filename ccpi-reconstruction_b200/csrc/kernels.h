@@ -13,7 +13,7 @@ int pb_fp_ctas(const Geom &g);
 int pb_backward(const Geom &g, const float *pix, float *vol, int mode, const Epi &e,
                 int *err, cudaStream_t st);
 int pb_bp_tiles(const Geom &g);
-int cb_prepare();
+int cb_prepare(const Geom &g);
 // band[i * ny + j] = the back projector's band rows [x, y) of voxel column
 // (i, j) (c2D.cpp:657-676); the cone back projectors read it as g.colband
 int cb_column_bands(const Geom &g, int2 *band, cudaStream_t st);
@@ -38,7 +38,7 @@ int cb_backward_scatter(const Geom &g, const float *pix, float *vol, int pre,
 // CTAs of the cone back projector (= its partial sums); its set-up, done by
 // cb_prepare.
 int cb_bp_parts(const Geom &g);
-int cb_bp_prepare();
+int cb_bp_prepare(const Geom &g);
 // The cone back projector accepts a sinogram pre-scaled by d_conv
 // (Epi::pre); cb_prescale writes that scaled copy.
 void cb_prescale(const Geom &g, const float *in, float *out, cudaStream_t st);
