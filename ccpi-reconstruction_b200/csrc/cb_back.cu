@@ -1124,9 +1124,11 @@ size_t small_smem(const Geom &g) {
 
 // Chunk height; warps per CTA.  Tall chunks spend less on ray set-up and
 // on rows that straddle two chunks; small problems need short chunks to reach
-// every SM.  Eight warps share a patch: CTAs of two or four, which would reach
-// more SMs, spend more on the copies (64^3 from 96 rows, 24 angles: 406 us, with two
-// warps 766).  32 slices, 8 warps and 17,000 patch floats
+// every SM.  Eight warps share a patch; CTAs of two or four reach more SMs but
+// copy more, so that they pay only with 32 slices (128^3 / 180 angles 7.2 ms with
+// four, 7.9 with eight) or where a voxel sees so many rays that few angles'
+// patches fit (64^2 x 256 with 25 rays per voxel 3.5 / 4.1 ms; with 6 rays 1.30
+// / 1.17; 8 slices, 96^3: 1.82 / 1.32).  32 slices, 8 warps and 17,000 patch floats
 // make two CTAs per SM (36 KB of accumulators, 4 KB of row tables and 66 KB
 // of patch each); 512^3: 617 ms, 660 ms with 24 slices, 831 ms with 16 slices
 // and three CTAs, 676 ms with one CTA of 16 warps.
@@ -1139,6 +1141,12 @@ TileShape tile_shape(const Geom &g) {
   t.nzc = (g.nz + t.zc - 1) / t.zc;
   t.wx = 2;
   t.wy = 4;
+  // detector columns and rows per voxel on the axis
+  const double mag = std::abs(g.cl / g.src[0]);
+  const bool dense = g.size[0] * mag * g.cipix * g.size[2] * mag * g.inv_pitch > 20.0;
+  while ((t.zc == 32 || (t.zc == 16 && dense)) && t.wy > 1 &&
+         warps * t.nzc < i64(296) * t.wx * t.wy)
+    t.wy /= 2;
   t.rcap = 512;
   t.cap = 17000;
   t.ntx = (g.nx + t.wx * kTileX - 1) / (t.wx * kTileX);
