@@ -52,8 +52,6 @@ struct Geom {
   int mid;                // first row above the source
   float dz0, inv_pitch, pitch_max; // dz[0], 1 / mean row step, largest row step
   int even_rows;          // every row within a quarter step of dz0 + v / inv_pitch
-  int even_cols;          // every column within 0.01 steps of its place in the even
-                          // spacing hpix[0], hpix[1] (cipix), which the axis is near
   const double2 *inv;     // na * nh: 1 / the ray's x and y spans (x = 0: the back
                           // projector takes no such ray, c2D.cpp:909-912)
   float neg0;             // -0.0f (see mul2_nz)
@@ -65,6 +63,11 @@ struct Geom {
   int tune_vw;            // parallel back projector: slices per lane (4, 8, 16)
   int tune_rpl;           // cone forward projector: rows per lane (2, 4, .. 12)
   int tune_scatter;       // cone back projector: 1 ray-driven scatter, 0 voxel gather
+  // ---- cone beam, continued
+  int even_cols;          // every column within 0.01 steps of its place in the even
+                          // spacing hpix[0], hpix[1] (cipix), which the axis is near
+  float row_edge;         // part of the volume's depth in which the outermost rows' rays
+                          // are past its ends (or in the last slice and a half)
 };
 
 // Epilogue operands shared by the fused projector epilogues.

@@ -308,6 +308,11 @@ int plan_create(const ccpi_geometry *gi, ccpi_plan **out) {
     for (int i = 0; i < nh; i++)
       if (!(std::abs((hp[i] - hp[0]) * g.cipix - i) <= 0.01))
         g.even_cols = 0;
+    const double end = 1.5 * g.size[2], depth = std::min(g.nx * g.size[0], g.ny * g.size[1]);
+    const double leave =
+        std::min((g.origin[2] + end - sz) / (vp[0] - sz),
+                 (g.origin[2] + nz * g.size[2] - end - sz) / (vp[nv - 1] - sz));
+    g.row_edge = float(((0.5 * depth - sx) / g.cl - leave) / (depth / g.cl));
     tables.add(g.dconv, dconv);
     tables.add(g.dz, dz);
     tables.add(g.iz, iz);
