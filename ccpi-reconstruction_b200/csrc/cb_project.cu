@@ -306,6 +306,32 @@ __device__ __forceinline__ void cb_fp_cells(const Geom &g, const float *alphas, 
   }
 }
 
+// cb_fp_cells for up to 32 rows, one per lane; side: the lane's side of the
+// source (-1 below, 1 above).  With two rows per lane half of them were idle
+// (512^2 x 8 from 16 rows, 60 angles: 7.9 ms; with one 6.5 ms).
+__device__ __forceinline__ float cb_fp_cells_one(const Geom &g, const float *alphas,
+                                                 const int *cells, int m1, const float *vol,
+                                                 const float *svz, float dz, float iz, int side) {
+  constexpr unsigned kMagic = 0x4b000000u; // bits of 2^23
+  const unsigned vz =
+      unsigned(__cvta_generic_to_shared(svz)) - 4 * kMagic + (side < 0 ? 0 : 4);
+  float acc = 0.0f;
+  for (int m = 1; m < m1; m++) {
+    const int cell = cells[m - 1];
+    if (cell < 0)
+      continue;
+    const float a0 = alphas[m - 1], a1 = alphas[m];
+    const char *col = reinterpret_cast<const char *>(vol + i64(cell) * g.nz) - 4ll * kMagic;
+    const float x = __fadd_rn(g.pzbz, __fmul_rn(__fmul_rn(a0, g.inv_dz), dz));
+    const unsigned k = __float_as_uint(__fadd_rz(x, 8388608.0f));
+    const float mz = fmin_ref(__fmul_rn(lds_f(at_smem(k, g.four, vz)), iz), a1);
+    const float *c = at_wide(k, g.four, col);
+    acc = __fadd_rn(acc, __fadd_rn(__fmul_rn(__ldg(c), __fsub_rn(mz, a0)),
+                                   __fmul_rn(__ldg(c + side), __fsub_rn(a1, mz))));
+  }
+  return acc;
+}
+
 // RPL = detector rows per lane per pass.  The np passes of 32 * RPL rows start
 // at row v0 <= 0, such that the first row above the source begins a pass or
 // the second half of one; rows outside [0, nv) act as a row at the source
@@ -364,6 +390,10 @@ __global__ void __launch_bounds__(kFpWarps * 32)
       // In [1, mfast) the regime search has shown that the lowest row's
       // slice index is >= 1 and the highest row's < nz - 1 (c2D.cpp:45-99),
       // so every row's k and its neighbour k -/+ 1 are inside the column.
+      if constexpr (RPL == 1) {
+        acc[0] = cb_fp_cells_one(g, alphas, cells, mfast, vol, svz, dzv[0], izv[0],
+                                 below[0] ? -1 : 1);
+      } else {
       float2 acc2[RPL / 2], dz2[RPL / 2], iz2[RPL / 2];
 #pragma unroll
       for (int q = 0; q < RPL; q += 2) {
@@ -383,6 +413,7 @@ __global__ void __launch_bounds__(kFpWarps * 32)
 #pragma unroll
       for (int q = 0; q < RPL; q++)
         acc[q] = (q & 1) ? acc2[q / 2].y : acc2[q / 2].x;
+      }
       for (int m = max(mfast, 1); m < n; m++) {
         const float a0 = alphas[m - 1], a1 = alphas[m];
         const int cell = cells[m - 1];
@@ -1056,6 +1087,8 @@ namespace {
 RowPasses cb_fp_rows(const Geom &g) {
   if (g.tune_rpl >= 2 && g.tune_rpl <= 12 && g.tune_rpl % 2 == 0)
     return row_passes(g, g.tune_rpl);
+  if (row_passes(g, 1).np == 1)
+    return row_passes(g, 1);
   RowPasses best = row_passes(g, 2);
   for (int r = 4; r <= 12; r += 2) {
     const RowPasses p = row_passes(g, r);
@@ -1079,7 +1112,8 @@ void launch_cb_fp(const Geom &g, const float *vol, float *pix, const Epi &e, con
   cb_fp_kernel<EPI, R, B><<<grid, kFpWarps * 32, smem, st>>>(g, vol, pix, e, hrange, cap, nb,  \
                                                              p.v0, p.np)
 #define CB_FP_RPL(B)                                                                       \
-  (p.rpl == 2   ? CB_FP_GO(2, B)                                                            \
+  (p.rpl == 1   ? CB_FP_GO(1, B)                                                            \
+   : p.rpl == 2 ? CB_FP_GO(2, B)                                                            \
    : p.rpl == 4 ? CB_FP_GO(4, B)                                                            \
    : p.rpl == 6 ? CB_FP_GO(6, B)                                                            \
    : p.rpl == 8 ? CB_FP_GO(8, B)                                                            \
@@ -1104,7 +1138,7 @@ int cb_prepare(const Geom &g) {
   (const void *)cb_fp_kernel<EPI_STORE, R, false>, (const void *)cb_fp_kernel<EPI_NORM, R, false>, \
       (const void *)cb_fp_kernel<EPI_SIRT, R, false>,                                       \
       (const void *)cb_fp_kernel<EPI_MLEM, R, false>, (const void *)cb_fp_kernel<EPI_STORE, R, true>
-  const void *fps[] = {CB_FP_ALL(2), CB_FP_ALL(4), CB_FP_ALL(6), CB_FP_ALL(8), CB_FP_ALL(10), CB_FP_ALL(12),
+  const void *fps[] = {CB_FP_ALL(1), CB_FP_ALL(2), CB_FP_ALL(4), CB_FP_ALL(6), CB_FP_ALL(8), CB_FP_ALL(10), CB_FP_ALL(12),
                        (const void *)cb_bp_scatter_edge<1, false>,
                        (const void *)cb_bp_scatter_edge<1, true>,
                        (const void *)cb_bp_scatter_edge<2, false>,
