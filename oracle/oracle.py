@@ -247,6 +247,10 @@ class quiet:
         return False
 
 
+class ReferenceMissing(FileNotFoundError):
+    """The reference's own build is not on this machine."""
+
+
 def reference_available():
     return os.path.exists(REF_SO)
 
@@ -255,7 +259,7 @@ def reference():
     global _ref
     if _ref is None:
         if not os.path.exists(REF_SO):
-            raise FileNotFoundError(f"{REF_SO} missing: run `make -C oracle ref`")
+            raise ReferenceMissing(f"{REF_SO} missing: run `make -C oracle ref`")
         lib = ctypes.CDLL(REF_SO)
         lib.ref_set_pad_factor.argtypes = [_c_dbl]
         lib.ref_pb_geometry.argtypes = [_c_int, _c_int, _c_int, _c_dbl, _c_int, _i32p, _f64p]

@@ -24,6 +24,16 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200)")
 
 
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_call(item):
+    """A test that comes to a call of the reference's own build where that
+    build is absent is skipped, not failed."""
+    outcome = yield
+    from oracle import ReferenceMissing
+    if outcome.excinfo is not None and issubclass(outcome.excinfo[0], ReferenceMissing):
+        outcome.force_exception(pytest.skip.Exception("the reference library is not built"))
+
+
 def golden(name):
     with np.load(os.path.join(GOLDEN, name + ".npz")) as z:
         return {k: z[k] for k in z.files}
