@@ -28,6 +28,7 @@ path; the time is the maximum over ranks.
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import math
 import os
@@ -90,19 +91,24 @@ def parse():
     return args
 
 
+def kernel_source_id(name):
+    """Identifies the code of one csrc file: a hash of its text without
+    comments and white space."""
+    with open(os.path.join(ROOT, "ccpi-reconstruction_b200", "csrc", name)) as f:
+        text = "".join(line.split("//")[0] for line in f)
+    return hashlib.sha256("".join(text.split()).encode()).hexdigest()[:16]
+
+
 def load_traffic(kernel):
     """DRAM bytes per launch of `kernel` on the full-size workload, from one
-    ncu capture of the same command (1-pass metrics), kept in profiles/."""
-    name = {"pb_fp": "pb_traffic_768x768x256.json", "pb_bp": "pb_traffic_768x768x256.json",
-            "cb_bp_tile": "cb_traffic_512cube.json", "cb_bp_scatter": "cb_traffic_512cube.json",
-            "cb_fp": "cb_traffic_512cube.json"}.get(kernel)
-    if name is None or (kernel.startswith("pb") and globals().get("NH") != 768):
+    ncu capture of the same command (1-pass metrics), kept in profiles/; None
+    where none was taken of the kernel's present source."""
+    name = "pb_traffic_768x768x256.json" if kernel.startswith("pb") else "cb_traffic_512cube.json"
+    if kernel.startswith("pb") and globals().get("NH") != 768:
         return None
-    try:
-        with open(os.path.join(ROOT, "profiles", name)) as f:
-            return float(json.load(f)["kernels"][kernel]["dram_bytes_per_launch"])
-    except Exception:
-        return None
+    with open(os.path.join(ROOT, "profiles", name)) as f:
+        k = json.load(f)["kernels"][kernel]
+    return float(k["dram_bytes_per_launch"]) if kernel_source_id(k["file"]) == k["source"] else None
 
 
 def pick_cone_bp(plan, choice):
