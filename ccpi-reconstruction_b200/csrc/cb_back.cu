@@ -20,12 +20,12 @@
 // reference's, in its order, with the same unfused roundings: the result is
 // the reference's bit for bit.
 //
-// Bound: instruction issue (59 % issue slots busy at 256^3, where the row
+// Bound: instruction issue (63 % issue slots busy at 256^3, where the row
 // loop takes half of a central tile's time, the copies and barriers a
 // quarter, ray set-up the rest).  Against one CTA per column with the rows
-// over its threads (now cb_bp_column, for small volumes), whose rows went
-// through shared memory to the voxels: 512^3 1245 -> 635 ms, 256^3 98.6 ->
-// 54.9 ms, 128^3 9.97 -> 7.2 ms.
+// over its threads (now cb_bp_column, for few columns), whose rows went
+// through shared memory to the voxels: 512^3 1245 -> 625 ms, 256^3 98.6 ->
+// 55 ms, 128^3 9.97 -> 7.3 ms.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -1130,7 +1130,7 @@ size_t small_smem(const Geom &g) {
 // patches fit (64^2 x 256 with 25 rays per voxel 3.5 / 4.1 ms; with 6 rays 1.30
 // / 1.17; 8 slices, 96^3: 1.82 / 1.32).  32 slices, 8 warps and 17,000 patch floats
 // make two CTAs per SM (36 KB of accumulators, 4 KB of row tables and 66 KB
-// of patch each); 512^3: 617 ms, 660 ms with 24 slices, 831 ms with 16 slices
+// of patch each); 512^3: 625 ms, 660 ms with 24 slices, 831 ms with 16 slices
 // and three CTAs, 676 ms with one CTA of 16 warps.
 TileShape tile_shape(const Geom &g) {
   TileShape t;

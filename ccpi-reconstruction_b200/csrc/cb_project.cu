@@ -12,15 +12,10 @@
 // distance.  Per row the additions happen in the reference's order with
 // unfused float operations, so the result matches the reference bit for bit.
 //
-// Backward (cone_beam::b2D, c2D.cpp:948-1119): voxel-column gather, the
-// reference's design.  One CTA owns one xy column; it finds, angle chunk by
-// angle chunk, every (angle, detector column) ray that crosses the column
-// with the reference's entry/exit alphas (c2D.cpp:788-946).  cb_bp_gather
-// then has each thread form its own voxels' sums over the rays' detector
-// rows (c2D.cpp:640-751) in the reference's order, bit for bit; columns
-// taller than 1024 voxels use cb_bp_kernel, whose warps spread rows into a
-// shared-memory accumulator with float atomics (unspecified order, equal to
-// the reference to float rounding).
+// Backward (cone_beam::b2D, c2D.cpp:948-1119): the ray-driven scatter, whose
+// additions into a voxel have no fixed order (two forms, see below), and the
+// plan's table of every voxel column's band.  The gathers in the reference's
+// order, bit for bit, are in cb_back.cu.
 #include <algorithm>
 
 #include "cb_common.cuh"
@@ -257,7 +252,7 @@ enum Side { BELOW = 0, ABOVE = 1, HALVES = 2 };
 // address formed per row, took 306 ms at 512^3 / 720 angles / 768^2; packed
 // sums (mul2_nz), int(x) by addition and immediate offsets 260 ms; addresses
 // as multiply-adds by a 4 the compiler cannot turn into shifts, which puts
-// them on the FMA pipe (26 % busy) instead of the ALU (50 %), 232 ms.
+// them on the FMA pipe instead of the ALU, 232 ms.
 __device__ __forceinline__ const float *at_wide(unsigned k, unsigned four, const char *c) {
   const float *r;
   asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(k), "r"(four), "l"(c));
@@ -497,11 +492,13 @@ __global__ void __launch_bounds__(kFpWarps * 32)
 // a1 - mz), and the row's value p = pix * d_conv times each weight goes to
 // the two voxels, with float atomics.  The order of the additions into a
 // voxel is not fixed: the result equals the reference's b2D to float
-// rounding, not bit for bit (cb_back.cu has that form).  `vol` must be zero on
-// entry; PRE: `pix` is already scaled by d_conv.
+// rounding, not bit for bit (cb_back.cu has that form).  Detector columns are
+// taken as even: off their even spacing b2D drops rays that its range of a
+// voxel column misses, which this does not.  `vol` must be zero on entry; PRE:
+// `pix` is already scaled by d_conv.
 //
-// Bound: instruction issue and the L2's atomics (54 % busy in the form before
-// this one, which issued twice the instructions).  Rows in lane-consecutive
+// Bound: instruction issue (82 % of the slots at 256^3), the L2 at 54 % of its
+// throughput with the atomics.  Rows in lane-consecutive
 // pairs, packed, and no atomic for a weight of zero: 512^3 501 -> 320 ms,
 // 256^3 30.9 -> 20.6 ms.  Without the test for zero weights 586 ms; with a
 // lane's pairs next to each other, so that an atomic instruction's slices

@@ -1,10 +1,11 @@
 // Parallel-beam Siddon projectors for sm_100a.
 //
-// Forward (parallel_beam::f2D, Core/src/p2D.cpp:468-611): ray-driven.  One
-// warp owns one ray (angle a, detector column h) and its lanes own detector
-// rows v, so every voxel-column read and every sinogram write is a
-// contiguous, coalesced row (float4 per lane when the layout allows).  The
-// xy walk is warp-uniform and is evaluated exactly as the reference does:
+// Forward (parallel_beam::f2D, Core/src/p2D.cpp:468-611): ray-driven.  A
+// warp owns one ray (angle a, detector column h), or several where the rows
+// do not fill it (pb_fp_groups), and lanes own rows or slices, so every
+// voxel-column read and every sinogram write is a contiguous, coalesced row
+// (float4 per lane when the layout allows).  The xy walk, a block per lane,
+// is evaluated exactly as the reference does:
 // the volume is cut into 32x32 xy blocks, blocks are visited in the
 // reference's (x-block, y-block) order, each block applies the reference's
 // detector-column range rule and is walked from its own entry point with
